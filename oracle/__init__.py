@@ -56,7 +56,7 @@ def build(ref: bool | None = None) -> None:
     """make -C oracle (and `make ref` when the reference sources are present)."""
     subprocess.run(["make", "-s", "-C", str(HERE)], check=True, capture_output=True)
     if ref is None:
-        ref = REFERENCE.exists()
+        ref = (REFERENCE / "CUDA").is_dir()  # an empty mount point holds no sources
     if ref:
         subprocess.run(["make", "-s", "-C", str(HERE), "ref", f"REFERENCE={REFERENCE}"], check=True,
                        capture_output=True)

@@ -6,6 +6,7 @@
 #include "capsp_internal.h"
 #include "graph_cache.h"
 
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <climits>
@@ -80,6 +81,13 @@ struct MixTable {
 void destroy_graph_exec(cudaGraphExec_t e) { cudaGraphExecDestroy(e); }
 typedef GraphCache<cudaGraphExec_t, destroy_graph_exec> Graphs;
 
+// Launch plan of the chain kernel over a view (kernels_chain.cuh)
+struct ChainPlan {
+    bool ok = false;
+    bool far = false;  // some entry reaches back beyond the ring
+    int ring = 0, warps = 0, slots = 0, entries = 0, lag = 0, ahead = 0;
+};
+
 // Level schedule of one row-driven view of the matrix (capsp_level_layout):
 // view 0 reads the stored arrays as rows (CSR rows; CSC columns, i.e. rows of
 // the transpose), view 1 their transpose, built on the host from the stored
@@ -92,6 +100,8 @@ struct RowView {
     bool narrow = false;  // levels narrower than ~4k rows on average
     int *d_perm = nullptr, *d_lptr = nullptr, *d_lidx = nullptr, *d_lsrc = nullptr, *d_dsrc = nullptr;
     void *d_lval = nullptr, *d_linv = nullptr;
+    int *d_lnear = nullptr;   // first near entry per position (chain.ok only)
+    ChainPlan chain;
     std::vector<int> h_lcum;  // lptr[k] + k: row-count prefix in position space (mix tables)
     // capsp_solve_host's b upload: highest b segment per 32 positions (kernel: b_group_seg)
     unsigned char *d_group_seg = nullptr;
@@ -178,6 +188,7 @@ struct capsp_handle_s {
     size_t l2_prev_limit = 0;  // persisting carve-out before this handle changed it
     size_t l2_window = 0;      // largest window the device accepts
     size_t l2_persist = 0;     // persisting carve-out this handle asked for
+    bool chain = true;      // narrow levels may take the chain kernel (capsp_hop_latency: no)
     int sched = CAPSP_SCHED_LEVEL;  // schedule of view 0; view 1 is always level-ordered
     RowView view[2];
     void *d_xp = nullptr;     // position-ordered publication scratch (both views)
@@ -222,6 +233,7 @@ static void free_handle(capsp_handle_t h)
         cudaFree(rv.d_lval);
         cudaFree(rv.d_linv);
         cudaFree(rv.d_group_seg);
+        cudaFree(rv.d_lnear);
     }
     cudaFree(h->d_xp);
     if (h->stage_stream)
@@ -326,6 +338,70 @@ static capsp_status_t transpose_structure(int n, int nnz, const int *ptr, const 
     return CAPSP_OK;
 }
 
+// Rows per level up to which the chain kernel is the faster one, per wave of
+// right-hand sides (a cluster each, 16 of them resident).  Measured on GB300 in
+// FP64, chain against row kernel: 8 rows per level (1,048,576 Zipf rows) 28.3
+// against 100.9 ms, 13 (2,003 rows) 27 against 137 us, 115 (40,000 rows of 3-12
+// dependencies) 191 against 461 us, 200 (20,000 rows) 57 against 92 us, 377
+// (60,000 rows) 171 against 147 us.
+constexpr long long kChainLevelRows = 256;
+constexpr int kChainWave = 16;
+
+// Plan of the chain kernel for a level layout, and the first near entry of
+// every position.
+//
+// Deep matrices (levels of less than two chunks) take 8 chain warps with two
+// slots each: more warps only add pollers to the chain (13 rows per level: 29
+// us with 8, 35 us with 16, 44 us with 4).  Wider levels are bound by the warps'
+// work per chunk and by the round trip that refills a slot: 16 warps (200 rows
+// per level: 93 us with 8, 73 us with 12, 60 us with 16) with four slots each
+// (54 us; three 62 us, two 82 us) while the near entries fit in slots that
+// small, else fewer slots.
+//
+// The ring holds the whole solve where the slots leave room for that, else
+// 4,096 values for deep matrices and 8,192 for wider levels, whose dependencies
+// reach further back in positions.  Half of a ring that wraps is the reach of
+// near entries; the other half lets the chain warps drift apart and marks
+// positions pending ahead of them.
+static ChainPlan plan_chain(int n, int levels, size_t vb, const int *lptr, const int *lidx, std::vector<int> &lnear)
+{
+    ChainPlan c;
+    if ((long long)n > kChainLevelRows * (long long)levels)
+        return c;
+    const bool deep = (long long)n < 64LL * (long long)levels;
+    c.ring = 1024;
+    while (c.ring < n && c.ring < (deep ? 16384 : 8192))
+        c.ring *= 2;
+    const bool all = c.ring >= n;
+    if (!all && deep)
+        c.ring = 4096;
+    const int span = all ? n : c.ring / 2;
+    lnear.resize((size_t)n);
+    const long long near_entries = capsp_near_split(n, lptr, lidx, 32, span, lnear.data());
+    const long long per_chunk = near_entries / ((n + 31) / 32);
+    c.far = near_entries < (long long)lptr[n];
+    // the chain block holds words, ring and slots, a feeder words and a staging
+    // area of a slot's size per warp
+    const int words = 1024 + 32, hdr = 32 * (int)(vb + 8);
+    const int shapes[4][2] = {{16, 4}, {16, 3}, {16, 2}, {8, 2}};  // warps, slots per warp
+    for (int k = deep ? 3 : 0; k < 4; ++k) {
+        c.warps = shapes[k][0];
+        c.slots = c.warps * shapes[k][1];
+        const int room = std::min((kChainSmem - words - c.ring * (int)vb) / c.slots, (kChainSmem - words) / kChainWarps);
+        c.entries = (room - hdr) / (int)(vb + 2) / 8 * 8;
+        if (per_chunk + per_chunk / 4 <= c.entries)
+            break;
+    }
+    if (!all) {
+        c.lag = (c.ring / 32 - span / 32 - 2) / 2;
+        c.ahead = c.lag + 1;
+    }
+    // rows whose near entries do not fit are walked in global memory: fine for
+    // a few chunks, not for the average one
+    c.ok = per_chunk <= c.entries;
+    return c;
+}
+
 // Build the level schedule of view v (host work O(nnz) plus one upload);
 // synchronous.
 static capsp_status_t build_view(capsp_handle_t h, int v)
@@ -391,6 +467,14 @@ static capsp_status_t build_view(capsp_handle_t h, int v)
         rv.h_lcum[k] = lptr[k] + k;
     rv.upper = upper;
     rv.levels = levels;
+    std::vector<int> lnear;
+    rv.chain = plan_chain(n, levels, vb, lptr.data(), lidx.data(), lnear);
+    cudaFree(rv.d_lnear);
+    rv.d_lnear = nullptr;
+    if (rv.chain.ok) {
+        CAPSP_CUDA(cudaMalloc(&rv.d_lnear, sizeof(int) * (size_t)n));
+        CAPSP_CUDA(cudaMemcpy(rv.d_lnear, lnear.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice));
+    }
     // levels narrower than ~4k rows: two resident warps per SM for the row
     // path by default (more rows in flight than a few levels only add pollers)
     rv.narrow = (long long)n < 4096LL * (long long)levels;
@@ -901,15 +985,9 @@ static void row_shape(capsp_handle_t h, int v, const Tuning &tn, int nrhs, int *
     }
 }
 
-// launch tuning of an operation with nrhs right-hand sides (autotuned choices
-// cover the plain solve)
-static Tuning current_tuning(capsp_handle_t h, Op op, int nrhs)
+// launch tuning of an operation
+static Tuning untuned(capsp_handle_t h, Op op)
 {
-    if (op == kOpSolve) {
-        auto it = h->tuned.find(nrhs);
-        if (it != h->tuned.end())
-            return it->second;
-    }
     const int v = view_of(h, op);
     const RowView &rv = h->view[v];
     Tuning t = h->tune;
@@ -933,9 +1011,20 @@ static Tuning current_tuning(capsp_handle_t h, Op op, int nrhs)
     case CAPSP_ALG_TWOPART: t.kind = kRowTwoPart; break;
     case CAPSP_ALG_MIX: t.kind = kRowMix; break;
     case CAPSP_ALG_WRTFST: t.kind = kRowWrtFst; break;
-    default: t.kind = -1; break;  // AUTO: decided from the mix table
+    default: t.kind = -1; break;  // AUTO: decided from the plan and the mix table
     }
     return t;
+}
+
+// ... with the autotuned choice of the plain solve, if there is one
+static Tuning current_tuning(capsp_handle_t h, Op op, int nrhs)
+{
+    if (op == kOpSolve) {
+        auto it = h->tuned.find(nrhs);
+        if (it != h->tuned.end())
+            return it->second;
+    }
+    return untuned(h, op);
 }
 
 // ---------------------------------------------------------------------------
@@ -957,6 +1046,62 @@ static capsp_status_t ensure_xp(capsp_handle_t h, int nrhs)
     return CAPSP_OK;
 }
 
+// whether a row-driven solve over view v takes the chain kernel: AUTO with the
+// default launch shape, outside the debug and L2-window modes
+static bool chain_selected(capsp_handle_t h, int v, const Tuning &tn, int nrhs)
+{
+    const RowView &rv = h->view[v];
+    const int waves = ((nrhs < 32 ? nrhs : 32) + kChainWave - 1) / kChainWave;
+    return view_level(h, v) && rv.chain.ok && tn.kind < 0 && tn.dflt && !h->border_explicit && h->chain &&
+           h->trace == nullptr && h->l2_mode == CAPSP_L2_HINTS &&
+           (long long)h->n * waves <= kChainLevelRows * (long long)rv.levels;
+}
+
+// chain kernel over view v, right-hand sides [0, nb) of b and x
+template <typename T>
+static capsp_status_t enqueue_chain(capsp_handle_t h, int v, const T *b, T *x, int nb, int64_t ld, bool first,
+                                    cudaStream_t st)
+{
+    const RowView &rv = h->view[v];
+    const ChainPlan &cp = rv.chain;
+    // far dependencies are polled in the publication vector, which starts
+    // all-pending; without them a single right-hand side needs one launch
+    if (cp.far)
+        CAPSP_CUDA(launch_fill_pending<T>((T *)h->d_xp, h->n, nb, nb, h->d_ticket, 1, first ? h->d_err : nullptr, st));
+    else if (first && nb > 1)
+        CAPSP_CUDA(cudaMemsetAsync(h->d_err, 0, sizeof(int) * 4, st));
+    ChainArgs<T> a;
+    a.perm = rv.d_perm;
+    a.lptr = rv.d_lptr;
+    a.lnear = rv.d_lnear;
+    a.lidx = rv.d_lidx;
+    a.lval = (const T *)rv.d_lval;
+    a.linv = (const T *)rv.d_linv;
+    a.xp = cp.far ? (T *)h->d_xp : nullptr;
+    a.b = b;
+    a.x = x;
+    a.ld = ld;
+    a.n = h->n;
+    a.nchunks = (h->n + 31) / 32;
+    a.ring = cp.ring;
+    a.warps = cp.warps;
+    a.slots = cp.slots;
+    a.entries = cp.entries;
+    a.lag = cp.lag;
+    a.ahead = cp.ahead;
+    a.reset_err = !cp.far && first && nb == 1;
+    a.err = h->d_err;
+    a.wait = h->wait;
+    a.stuck_row = h->stuck_row;
+    const bool prof = h->profiling && first;
+    if (prof)
+        CAPSP_CUDA(cudaEventRecord(h->ev_k0, st));
+    CAPSP_CUDA(launch_chain_solve<T>(a, nb, st));
+    if (prof)
+        CAPSP_CUDA(cudaEventRecord(h->ev_k1, st));
+    return CAPSP_OK;
+}
+
 // row-driven solve over view v
 template <typename T>
 static capsp_status_t enqueue_rows(capsp_handle_t h, int v, const T *b, T *x, int nrhs, int64_t ld,
@@ -970,6 +1115,10 @@ static capsp_status_t enqueue_rows(capsp_handle_t h, int v, const T *b, T *x, in
     }
     for (int r0 = 0; r0 < nrhs; r0 += 32) {
         const int nb = nrhs - r0 < 32 ? nrhs - r0 : 32;
+        if (chain_selected(h, v, tn, nrhs)) {
+            CAPSP_TRY(enqueue_chain<T>(h, v, b + r0, x + r0, nb, ld, r0 == 0, st));
+            continue;
+        }
         int kind = tn.kind;
         MixTable *mt = nullptr;
         // AUTO with 8+ lanes per row: a heavy row would get only 32/G slices,
@@ -1230,7 +1379,7 @@ static capsp_status_t prepare(capsp_handle_t h, int nrhs, Op op)
         CAPSP_TRY(ensure_xp(h, nrhs));
     }
     const Tuning tn = current_tuning(h, op, nrhs);
-    if (tn.kind == kRowMix || tn.kind < 0) {
+    if ((tn.kind == kRowMix || tn.kind < 0) && !chain_selected(h, v, tn, nrhs)) {
         MixTable *mt = nullptr;
         for (int r0 = 0; r0 < nrhs; r0 += 32) {
             const int nb = nrhs - r0 < 32 ? nrhs - r0 : 32;
@@ -1369,7 +1518,7 @@ extern "C" capsp_status_t capsp_solve_host(capsp_handle_t h, const void *b_host,
     const int v = view_of(h, kOpSolve);
     const long long nseg_want = ((long long)h->n + kSegmentRowsMin - 1) / kSegmentRowsMin;
     const Tuning tn = current_tuning(h, kOpSolve, nrhs);
-    const bool progressive = !column_driven(h, kOpSolve) && view_level(h, v) && nseg_want >= 2 &&
+    const bool progressive = !chain_selected(h, v, tn, nrhs) && !column_driven(h, kOpSolve) && view_level(h, v) && nseg_want >= 2 &&
                              row_hostio_supported(tn.kind < 0 ? kRowWrtFst : tn.kind, tn.R, nrhs) &&
                              wait_value32() != nullptr && pinned_alias(x_host, h->device) != nullptr;
     if (!progressive) {
@@ -1504,6 +1653,9 @@ extern "C" capsp_status_t capsp_autotune(capsp_handle_t h, const void *b, void *
         const bool allow_thread = alg == CAPSP_ALG_AUTO || alg == CAPSP_ALG_WRTFST;
         const bool allow_mix = alg == CAPSP_ALG_AUTO || alg == CAPSP_ALG_MIX;
         const int bpss[3] = {1, 2, 0};
+        const Tuning base = untuned(h, kOpSolve);
+        if (chain_selected(h, v, base, nrhs))
+            cands.push_back(base);
         if (allow_thread) {
             // the default launch shape first: the search never ends worse
             cands.push_back({kRowWrtFst, 1, 256, 1, h->border, true});
@@ -1713,6 +1865,13 @@ extern "C" capsp_status_t capsp_get_info(capsp_handle_t h, capsp_info_t *info)
             info->element_occupy = mit->second.eo;
             if (alg == CAPSP_ALG_AUTO)
                 alg = mit->second.wo > 0.0 ? CAPSP_ALG_MIX : CAPSP_ALG_WRTFST;
+        } else if (chain_selected(h, v, tn, 1)) {
+            // the chain kernel needs no selector table on the device; report
+            // the row kernels' choice for this matrix
+            std::vector<int> table((size_t)h->n + 2);
+            info->mix_len = capsp_mix_table(h->n, h->view[v].h_lcum.data(), 0, 32, tn.border, table.data(),
+                                            &info->warp_occupy, &info->element_occupy);
+            alg = info->warp_occupy > 0.0 ? CAPSP_ALG_MIX : CAPSP_ALG_WRTFST;
         }
         info->algorithm = alg;
     }
@@ -1749,6 +1908,7 @@ extern "C" capsp_status_t capsp_hop_latency(int n, int stride, int dtype, float 
     const void *val = dtype == CAPSP_R_64F ? (const void *)v64.data() : (const void *)v32.data();
     capsp_handle_t h = nullptr;
     CAPSP_TRY(capsp_analyse(n, nnz, ptr.data(), idx.data(), val, dtype, CAPSP_FMT_CSR, CAPSP_LOWER, 0, &h));
+    h->chain = false;  // the probe measures the row kernel's hop
     const size_t vb = dtype == CAPSP_R_64F ? 8 : 4;
     void *d_b = nullptr, *d_x = nullptr;
     std::vector<double> ones64((size_t)n, 1.0);

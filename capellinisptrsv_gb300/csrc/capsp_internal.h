@@ -66,6 +66,42 @@ struct RowArgs {
     const unsigned char *b_group_seg;
 };
 
+// The chain kernel (kernels_chain.cuh): a cluster of kChainBlocks blocks of
+// kChainWarps warps per right-hand side.
+constexpr int kChainBlocks = 8;
+constexpr int kChainWarps = 16;
+constexpr int kChainSmem = 232448;  // shared memory a block may take (227 KB)
+
+// Arguments of the chain solve: the level schedule (as RowArgs) and, per
+// position, lnear[p] = the first entry within reach of the ring of recent
+// values in shared memory (the entries before it are far: folded by the
+// feeders through the publication vector).
+template <typename T>
+struct ChainArgs {
+    const int *perm;
+    const int *lptr;
+    const int *lnear;
+    const int *lidx;
+    const T *lval;
+    const T *linv;
+    T *xp;  // publication vector, right-hand side r at xp + r * n (nullptr: no far entries)
+    const T *b;
+    T *x;
+    long long ld;
+    int n;
+    int nchunks;  // of 32 positions
+    int ring;     // values in the ring (a power of two)
+    int warps;    // warps of the chain block that take chunks
+    int slots;    // fed chunks in shared memory, a multiple of `warps`
+    int entries;  // near entries a slot holds (a multiple of 8)
+    int lag;      // chunks that the warps may drift apart (0: the ring holds the whole solve)
+    int ahead;    // chunks ahead of its own that a warp marks pending
+    int reset_err;
+    int *err;
+    WaitCfg wait;
+    int stuck_row;
+};
+
 // Arguments of the column-driven solve (SyncFree CSC kernel, and the
 // transpose solve that walks CSR rows as columns of the transpose).
 template <typename T>
@@ -121,6 +157,10 @@ inline bool row_hostio_supported(int kind, int rows_per_thread, int nrhs)
 template <typename T>
 cudaError_t launch_row_solve(const RowArgs<T> &a, int kind, int rows_per_thread, int block,
                              int blocks_per_sm, int num_sms, bool regcap, bool stage, cudaStream_t st);
+
+// nrhs clusters: right-hand side r at b + r, x + r (row stride ld) and xp + r * n
+template <typename T>
+cudaError_t launch_chain_solve(const ChainArgs<T> &a, int nrhs, cudaStream_t st);
 
 template <typename T>
 cudaError_t launch_col_solve(const ColArgs<T> &a, int block, int blocks_per_sm, int num_sms,

@@ -440,6 +440,30 @@ int capsp_level_layout(int n, const int *ptr, const int *idx, int upper, const i
     return bad ? -1 : 0;
 }
 
+/* First entry of every position whose dependency lies at most `span` positions
+ * before the start of the position's group of `group_rows` (a group's rows are
+ * solved together); the dependencies of a position ascend.  Returns how many
+ * entries of the layout are near in that sense. */
+long long capsp_near_split(int n, const int *dep_ptr, const int *dep_idx, int group_rows, int span, int *first_near)
+{
+    long long near_entries = 0;
+#pragma omp parallel for schedule(static, 8192) reduction(+ : near_entries)
+    for (int k = 0; k < n; ++k) {
+        const int reach = k / group_rows * group_rows - span;
+        int lo = dep_ptr[k], hi = dep_ptr[k + 1];
+        while (lo < hi) {
+            const int mid = lo + (hi - lo) / 2;
+            if (dep_idx[mid] < reach)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        first_near[k] = lo;
+        near_entries += dep_ptr[k + 1] - lo;
+    }
+    return near_entries;
+}
+
 void capsp_indegree(int n, int nnz, const int *idx, int *indeg)
 {
     memset(indeg, 0, sizeof(int) * (size_t)(n > 0 ? n : 1));

@@ -1,5 +1,6 @@
 // Explicit instantiation of the solve kernels for VALUE_TYPE float.  One
 // translation unit per value type so the two compile in parallel.
+#include "kernels_chain.cuh"
 #include "kernels_col.cuh"
 #include "kernels_row.cuh"
 
@@ -7,6 +8,7 @@ namespace capsp {
 
 template cudaError_t launch_row_solve<float>(const RowArgs<float> &, int, int, int, int, int, bool, bool,
                                                 cudaStream_t);
+template cudaError_t launch_chain_solve<float>(const ChainArgs<float> &, int, cudaStream_t);
 template cudaError_t launch_col_solve<float>(const ColArgs<float> &, int, int, int, cudaStream_t);
 template cudaError_t launch_fill_pending<float>(float *, int, int, long long, unsigned *, int, int *,
                                               cudaStream_t);

@@ -1,5 +1,6 @@
 // Explicit instantiation of the solve kernels for VALUE_TYPE double.  One
 // translation unit per value type so the two compile in parallel.
+#include "kernels_chain.cuh"
 #include "kernels_col.cuh"
 #include "kernels_row.cuh"
 
@@ -7,6 +8,7 @@ namespace capsp {
 
 template cudaError_t launch_row_solve<double>(const RowArgs<double> &, int, int, int, int, int, bool, bool,
                                                 cudaStream_t);
+template cudaError_t launch_chain_solve<double>(const ChainArgs<double> &, int, cudaStream_t);
 template cudaError_t launch_col_solve<double>(const ColArgs<double> &, int, int, int, cudaStream_t);
 template cudaError_t launch_fill_pending<double>(double *, int, int, long long, unsigned *, int, int *,
                                               cudaStream_t);

@@ -552,6 +552,15 @@ def level_layout(n, rowptr, colidx, order, position, upper: bool = False):
     return dep_ptr, dep_idx[:nd], dep_src[:nd], diag_src
 
 
+def near_split(n, dep_ptr, dep_idx, span: int, group_rows: int = 32):
+    """Where each position's near entries begin (level_layout arrays) -> (first_near, near entries)."""
+    dep_ptr = np.ascontiguousarray(dep_ptr, np.int32)
+    dep_idx = np.ascontiguousarray(dep_idx, np.int32)
+    first = np.empty(n, np.int32)
+    near = N.lib.capsp_near_split(int(n), _ptr(dep_ptr), _ptr(dep_idx), int(group_rows), int(span), _ptr(first))
+    return first, int(near)
+
+
 def transpose_structure(n, rowptr, colidx):
     """The structure transposed -> (tptr, tidx, src): new row j lists the stored
     rows holding index j, ascending; src maps new entries to stored ones."""

@@ -80,7 +80,9 @@ typedef enum capsp_uplo {
  * algorithms below apply to both; CAPSP_ALG_SYNCFREE_CSC instead solves the
  * other orientation column by column on the stored arrays. */
 typedef enum capsp_algorithm {
-    CAPSP_ALG_AUTO = 0,        /* mix when the selector finds heavy row groups, else WRTFST */
+    CAPSP_ALG_AUTO = 0,        /* level schedule with levels of up to 256 rows on average: the chain kernel
+                                  (the dependency chain inside one SM); else mix when the selector
+                                  finds heavy row groups, else WRTFST */
     CAPSP_ALG_WRTFST = 1,      /* thread per row, write-first (CUDA/ourWrtFst) */
     CAPSP_ALG_TWOPART = 2,     /* thread per row, out-of-warp then in-warp phases (CUDA/our2Part) */
     CAPSP_ALG_MIX = 3,         /* thread or warp per row by nnz/row of 32-row groups (CUDA/mix) */
@@ -479,6 +481,13 @@ int capsp_transpose_structure(int n, int nnz, const int *ptr, const int *idx, in
 int capsp_level_layout(int n, const int *ptr, const int *idx, int upper, const int *order,
                        const int *position, int *dep_ptr, int *dep_idx, int *dep_src,
                        int *diag_src);
+
+/* Where each position's near entries begin in such a layout: the first one
+ * whose dependency lies at most `span` positions before the start of the
+ * position's group of group_rows consecutive positions.  first_near: n.
+ * Returns the number of near entries of all positions. */
+long long capsp_near_split(int n, const int *dep_ptr, const int *dep_idx, int group_rows, int span,
+                           int *first_near);
 
 /* In-degree analyser: histogram of idx (CUDA/SyncFree_csc/spts_syncfree_cuda2.h:10-21,
  * openCL/SynFree_csc/sptrsv_syncfree_serialref.h:6-23). */

@@ -124,6 +124,8 @@ _SIGS = {
     "capsp_level_schedule": (I, [I, P, P, I, P, P, P]),
     "capsp_level_layout": (I, [I, P, P, I, P, P, P, P, P, P]),
     "capsp_near_split": (C.c_longlong, [I, P, P, I, I, P]),
+    "capsp_stream_slices": (I, [I, P]),
+    "capsp_stream_layout": (C.c_longlong, [I, P, P, I, P, P]),
     "capsp_transpose_structure": (I, [I, I, P, P, P, P, P]),
     "capsp_validate": (I, [I, I, P, P, I, I, C.c_char_p, I]),
     "read_mtx_f64": (I, [C.c_char_p, IP, IP, IP, C.POINTER(P), C.POINTER(P), C.POINTER(P)]),

@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <tuple>
@@ -88,6 +89,20 @@ struct ChainPlan {
     int ring = 0, warps = 0, slots = 0, entries = 0, lag = 0, ahead = 0;
 };
 
+// Layout of the stream kernel over a view (kernels_stream.cuh); built at analysis
+// where every solve takes it, else before the first solve that does
+struct StreamPlan {
+    bool tried = false;  // built, or found unsuitable
+    bool ok = false;
+    int nslices = 0;
+    void *d_all = nullptr;  // the arrays below
+    int *d_pos = nullptr, *d_row = nullptr, *d_idx = nullptr, *d_src = nullptr;
+    int2 *d_slice = nullptr;
+    void *d_val = nullptr, *d_linv = nullptr;
+    void *d_pub = nullptr;  // publication vector
+    int pub_cap = 0;        // values per position it holds
+};
+
 // Level schedule of one row-driven view of the matrix (capsp_level_layout):
 // view 0 reads the stored arrays as rows (CSR rows; CSC columns, i.e. rows of
 // the transpose), view 1 their transpose, built on the host from the stored
@@ -97,11 +112,14 @@ struct RowView {
     bool built = false;
     int upper = 0;        // its rows are upper-triangular (diagonal first)
     int levels = 0;
+    int longest = 0;      // dependencies of its longest row
     bool narrow = false;  // levels narrower than ~4k rows on average
     int *d_perm = nullptr, *d_lptr = nullptr, *d_lidx = nullptr, *d_lsrc = nullptr, *d_dsrc = nullptr;
     void *d_lval = nullptr, *d_linv = nullptr;
     int *d_lnear = nullptr;   // first near entry per position (chain.ok only)
     ChainPlan chain;
+    StreamPlan stream;
+    std::vector<int> h_levels;  // first position of every level, and n
     std::vector<int> h_lcum;  // lptr[k] + k: row-count prefix in position space (mix tables)
     // capsp_solve_host's b upload: highest b segment per 32 positions (kernel: b_group_seg)
     unsigned char *d_group_seg = nullptr;
@@ -188,7 +206,7 @@ struct capsp_handle_s {
     size_t l2_prev_limit = 0;  // persisting carve-out before this handle changed it
     size_t l2_window = 0;      // largest window the device accepts
     size_t l2_persist = 0;     // persisting carve-out this handle asked for
-    bool chain = true;      // narrow levels may take the chain kernel (capsp_hop_latency: no)
+    bool row_kernels_only = false;  // capsp_hop_latency; capsp_solve_host while b or x is on its way
     int sched = CAPSP_SCHED_LEVEL;  // schedule of view 0; view 1 is always level-ordered
     RowView view[2];
     void *d_xp = nullptr;     // position-ordered publication scratch (both views)
@@ -199,6 +217,13 @@ struct capsp_handle_s {
 };
 
 static bool diag_last_of(int format, int uplo) { return (format == CAPSP_FMT_CSR) == (uplo == CAPSP_LOWER); }
+
+static void free_stream(StreamPlan &sp)
+{
+    cudaFree(sp.d_all);
+    cudaFree(sp.d_pub);
+    sp = StreamPlan();
+}
 
 static void free_handle(capsp_handle_t h)
 {
@@ -234,6 +259,7 @@ static void free_handle(capsp_handle_t h)
         cudaFree(rv.d_linv);
         cudaFree(rv.d_group_seg);
         cudaFree(rv.d_lnear);
+        free_stream(rv.stream);
     }
     cudaFree(h->d_xp);
     if (h->stage_stream)
@@ -283,11 +309,45 @@ static capsp_status_t refresh_inv_diag(capsp_handle_t h)
     return CAPSP_OK;
 }
 
+// the arrays of a view's stream layout and of the view
+template <typename T>
+static StreamBuild<T> stream_arrays(const RowView &rv, const StreamPlan &sp)
+{
+    StreamBuild<T> a;
+    a.slice = sp.d_slice;
+    a.npos = 8LL * sp.nslices;
+    a.pos = sp.d_pos;
+    a.place = (int *)sp.d_linv;
+    a.perm = rv.d_perm;
+    a.lptr = rv.d_lptr;
+    a.lidx = rv.d_lidx;
+    a.lsrc = rv.d_lsrc;
+    a.lval = (const T *)rv.d_lval;
+    a.view_linv = (const T *)rv.d_linv;
+    a.row = sp.d_row;
+    a.idx = sp.d_idx;
+    a.src = sp.d_src;
+    a.val = (T *)sp.d_val;
+    a.linv = (T *)sp.d_linv;
+    return a;
+}
+
 // level-schedule values of one built view from the handle's current values, on `st`
 static capsp_status_t launch_view_refresh(capsp_handle_t h, const RowView &rv, int *bad, cudaStream_t st)
 {
     if (!rv.built)
         return CAPSP_OK;
+    if (rv.stream.ok) {
+        if (h->dtype == CAPSP_R_64F)
+            CAPSP_CUDA(launch_stream_values<double>(stream_arrays<double>(rv, rv.stream), rv.d_dsrc,
+                                                    (const double *)h->d_val, (double *)rv.d_linv,
+                                                    (double *)rv.d_lval, bad, st));
+        else
+            CAPSP_CUDA(launch_stream_values<float>(stream_arrays<float>(rv, rv.stream), rv.d_dsrc,
+                                                   (const float *)h->d_val, (float *)rv.d_linv, (float *)rv.d_lval,
+                                                   bad, st));
+        return CAPSP_OK;
+    }
     if (h->dtype == CAPSP_R_64F)
         CAPSP_CUDA(launch_level_values<double>(rv.d_lptr, rv.d_lsrc, rv.d_dsrc, h->n, (const double *)h->d_val,
                                                (double *)rv.d_lval, (double *)rv.d_linv, bad, st));
@@ -402,6 +462,69 @@ static ChainPlan plan_chain(int n, int levels, size_t vb, const int *lptr, const
     return c;
 }
 
+// Rows per level from which the stream kernel is the faster one whatever the
+// number of right-hand sides (stream_wanted)
+constexpr long long kStreamAnyRows = 12288;
+
+// Layout of the stream kernel for a view whose level layout is built
+// (rv.stream.ok, unless padding would double the entries); synchronous.
+static capsp_status_t build_stream(capsp_handle_t h, RowView &rv)
+{
+    if (rv.stream.tried)
+        return CAPSP_OK;
+    h->graphs.invalidate();
+    StreamPlan sp;
+    sp.tried = true;
+    sp.nslices = capsp_stream_slices(rv.levels, rv.h_levels.data());
+    const size_t ns = sp.nslices > 0 ? (size_t)sp.nslices : 0;
+    std::unique_ptr<int[]> rec(new (std::nothrow) int[2 * ns + 1]), pos(new (std::nothrow) int[8 * ns + 1]);
+    if (!rec || !pos)
+        return fail(CAPSP_ERR_OOM, "host allocation failed while laying out slices");
+    long long entries = LLONG_MAX;
+    if (sp.nslices > 0)
+        entries = capsp_stream_layout(rv.levels, rv.h_levels.data(), rv.h_lcum.data(), 1, rec.get(), pos.get());
+    if (entries < 0)
+        return fail(CAPSP_ERR_OOM, "host allocation failed while laying out slices");
+    if (entries > INT_MAX || entries > 2 * ((long long)h->nnz - h->n) + 256LL * rv.levels) {
+        rv.stream = sp;
+        return CAPSP_OK;
+    }
+    // one allocation: slices, positions, rows, 1/diagonals (holding `place`, an int
+    // per view position, while the layout is built), indices, sources, values
+    const size_t ne = (size_t)entries, np = 8 * ns, vb = h->vbytes;
+    const size_t bytes[7] = {sizeof(int2) * ns, 4 * np, 4 * np, vb * np, 4 * ne, 4 * ne, vb * ne};
+    size_t at[8] = {0};
+    for (int k = 0; k < 7; ++k)
+        at[k + 1] = at[k] + (bytes[k] + 255) / 256 * 256;
+    CAPSP_CUDA(cudaMalloc(&sp.d_all, at[7]));
+    char *base = (char *)sp.d_all;
+    sp.d_slice = (int2 *)(base + at[0]);
+    sp.d_pos = (int *)(base + at[1]);
+    sp.d_row = (int *)(base + at[2]);
+    sp.d_linv = base + at[3];
+    sp.d_idx = (int *)(base + at[4]);
+    sp.d_src = (int *)(base + at[5]);
+    sp.d_val = base + at[6];
+    cudaError_t e = cudaMemcpy(sp.d_slice, rec.get(), bytes[0], cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = cudaMemcpy(sp.d_pos, pos.get(), bytes[1], cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = cudaDeviceSynchronize();  // a refresh of the view may be under way on another stream
+    if (e == cudaSuccess)
+        e = h->dtype == CAPSP_R_64F ? launch_stream_layout<double>(stream_arrays<double>(rv, sp), 0)
+                                    : launch_stream_layout<float>(stream_arrays<float>(rv, sp), 0);
+    if (e == cudaSuccess)
+        e = cudaDeviceSynchronize();
+    if (e != cudaSuccess) {
+        free_stream(sp);
+        return fail(e == cudaErrorMemoryAllocation ? CAPSP_ERR_OOM : CAPSP_ERR_CUDA, "stream layout failed: %s",
+                    cudaGetErrorString(e));
+    }
+    sp.ok = true;
+    rv.stream = sp;
+    return CAPSP_OK;
+}
+
 // Build the level schedule of view v (host work O(nnz) plus one upload);
 // synchronous.
 static capsp_status_t build_view(capsp_handle_t h, int v)
@@ -425,7 +548,8 @@ static capsp_status_t build_view(capsp_handle_t h, int v)
     std::vector<int> order((size_t)n), position((size_t)n), lptr((size_t)n + 1), dsrc((size_t)n);
     const size_t ndeps = (size_t)nnz - (size_t)n;
     std::vector<int> lidx(ndeps > 0 ? ndeps : 1), lsrc(ndeps > 0 ? ndeps : 1);
-    const int levels = capsp_level_schedule(n, vptr, vidx, upper, order.data(), position.data(), nullptr);
+    std::vector<int> level_start((size_t)n + 2);
+    const int levels = capsp_level_schedule(n, vptr, vidx, upper, order.data(), position.data(), level_start.data());
     if (levels < 0)
         return fail(CAPSP_ERR_OOM, "host allocation failed while building the level schedule");
     if (capsp_level_layout(n, vptr, vidx, upper, order.data(), position.data(), lptr.data(), lidx.data(),
@@ -465,6 +589,9 @@ static capsp_status_t build_view(capsp_handle_t h, int v)
     rv.h_lcum.resize((size_t)n + 1);
     for (int k = 0; k <= n; ++k)
         rv.h_lcum[k] = lptr[k] + k;
+    rv.longest = 0;
+    for (int k = 0; k < n; ++k)
+        rv.longest = std::max(rv.longest, lptr[(size_t)k + 1] - lptr[(size_t)k]);
     rv.upper = upper;
     rv.levels = levels;
     std::vector<int> lnear;
@@ -475,6 +602,8 @@ static capsp_status_t build_view(capsp_handle_t h, int v)
         CAPSP_CUDA(cudaMalloc(&rv.d_lnear, sizeof(int) * (size_t)n));
         CAPSP_CUDA(cudaMemcpy(rv.d_lnear, lnear.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice));
     }
+    free_stream(rv.stream);
+    rv.h_levels.assign(level_start.begin() + 1, level_start.begin() + levels + 2);
     // levels narrower than ~4k rows: two resident warps per SM for the row
     // path by default (more rows in flight than a few levels only add pollers)
     rv.narrow = (long long)n < 4096LL * (long long)levels;
@@ -492,6 +621,8 @@ static capsp_status_t build_view(capsp_handle_t h, int v)
         return fail(CAPSP_ERR_CUDA, "level-schedule upload failed");
     if (bad != INT_MAX)
         return fail(CAPSP_ERR_INVALID, "zero or non-finite diagonal at schedule position %d", bad);
+    if (rv.longest <= 64 && (long long)n >= kStreamAnyRows * (long long)levels)
+        return build_stream(h, rv);
     return CAPSP_OK;
 }
 
@@ -1046,15 +1177,121 @@ static capsp_status_t ensure_xp(capsp_handle_t h, int nrhs)
     return CAPSP_OK;
 }
 
+// layout and publication scratch of the stream kernel over view v, whose level
+// layout is built
+static capsp_status_t ensure_stream(capsp_handle_t h, int v, int nrhs)
+{
+    CAPSP_TRY(build_stream(h, h->view[v]));
+    StreamPlan &sp = h->view[v].stream;
+    const int want = lanes_for_rhs(nrhs < 32 ? nrhs : 32);
+    if (sp.ok && sp.pub_cap < want) {
+        h->graphs.invalidate();  // captured stream solves point at the old scratch
+        cudaFree(sp.d_pub);
+        sp.d_pub = nullptr;
+        sp.pub_cap = 0;
+        CAPSP_CUDA(cudaMalloc(&sp.d_pub, h->vbytes * 8 * (size_t)sp.nslices * (size_t)want));
+        sp.pub_cap = want;
+    }
+    return CAPSP_OK;
+}
+
 // whether a row-driven solve over view v takes the chain kernel: AUTO with the
 // default launch shape, outside the debug and L2-window modes
 static bool chain_selected(capsp_handle_t h, int v, const Tuning &tn, int nrhs)
 {
     const RowView &rv = h->view[v];
     const int waves = ((nrhs < 32 ? nrhs : 32) + kChainWave - 1) / kChainWave;
-    return view_level(h, v) && rv.chain.ok && tn.kind < 0 && tn.dflt && !h->border_explicit && h->chain &&
+    return view_level(h, v) && rv.chain.ok && tn.kind < 0 && tn.dflt && !h->border_explicit && !h->row_kernels_only &&
            h->trace == nullptr && h->l2_mode == CAPSP_L2_HINTS &&
            (long long)h->n * waves <= kChainLevelRows * (long long)rv.levels;
+}
+
+// Whether a row-driven solve over view v would take the stream kernel (as above;
+// the debug hook of a row that never publishes stays with the row kernels).
+// The row kernels follow a chain of dependencies faster, the stream kernel gets
+// through more rows.  Measured on GB300, time of the row kernel / time of the
+// stream kernel:
+//   1 RHS: FP64 0.87 at 5.9k rows per level, 1.03 at 12k, 1.25 at 14k, 1.36 at 47k;
+//          FP32 0.92, -, 1.40, 1.42
+//   2 RHS: FP64 0.91 at 5.9k, 1.47 at 14k, 1.74 at 47k; FP32 1.00, 1.51, 1.86
+//   4 and more, FP32: 1.04 to 3.0 from 700 rows per level on
+//   4 and more, FP64: by the rows' length.  5 to 8 entries on average (12 fit a
+//          lane, 8 a lane of the row kernel): 1.05 to 1.24 from 700 rows per level
+//          on.  Shorter: 1.03 at 4.6k row-columns per level, 0.96 at 11k, 1.17 at
+//          23k, 1.10 to 1.49 above.  Longer: 0.94 at 6k, 1.10 at 12k.
+static bool stream_wanted(capsp_handle_t h, int v, const Tuning &tn, int nrhs)
+{
+    const RowView &rv = h->view[v];
+    if (!view_level(h, v) || !rv.built || tn.kind >= 0 || !tn.dflt || h->border_explicit || h->trace != nullptr ||
+        h->stuck_row >= 0 || h->l2_mode != CAPSP_L2_HINTS || h->row_kernels_only)
+        return false;
+    if (rv.longest > 64)  // such rows want a warp (the mixed row kernel)
+        return false;
+    const long long rows = (long long)h->n / rv.levels;  // per level
+    const int cols = lanes_for_rhs(nrhs < 32 ? nrhs : 32);
+    if (rows >= kStreamAnyRows)
+        return true;
+    if (rows < kChainLevelRows || cols == 1)
+        return false;
+    if (cols == 2)
+        return rows >= 8192;
+    if (h->dtype == CAPSP_R_32F)
+        return true;
+    const long long entries = (long long)h->nnz - h->n;
+    if (entries > 8LL * h->n)
+        return rows * cols >= 10240;
+    return entries > 5LL * h->n || rows * cols >= 16384;
+}
+
+static bool stream_selected(capsp_handle_t h, int v, const Tuning &tn, int nrhs)
+{
+    return h->view[v].stream.ok && stream_wanted(h, v, tn, nrhs);
+}
+
+// stream kernel over view v, right-hand sides [0, nb) of b and x
+template <typename T>
+static capsp_status_t enqueue_stream(capsp_handle_t h, int v, const T *b, T *x, int nb, int64_t ld, bool first,
+                                    cudaStream_t st)
+{
+    const StreamPlan &sp = h->view[v].stream;
+    const int cols = lanes_for_rhs(nb);
+    CAPSP_CUDA(launch_fill_pending<T>((T *)sp.d_pub, 8 * sp.nslices, cols, cols, h->d_ticket, 3,
+                                      first ? h->d_err : nullptr, st));
+    StreamArgs<T> a;
+    a.slice = sp.d_slice;
+    a.npos = 8LL * sp.nslices;
+    a.row = sp.d_row;
+    a.linv = (const T *)sp.d_linv;
+    a.idx = sp.d_idx;
+    a.val = (const T *)sp.d_val;
+    a.xp = (T *)sp.d_pub;
+    a.b = b;
+    a.x = x;
+    a.ld = ld;
+    a.nrhs = nb;
+    a.words = h->d_ticket;
+    a.err = h->d_err;
+    a.wait = h->wait;
+    const bool prof = h->profiling && first;
+    if (prof)
+        CAPSP_CUDA(cudaEventRecord(h->ev_k0, st));
+    // Rows of 5 to 8 entries on average take the build with 12 in one go
+    // (2,048 banded systems of 3-12 entries, 1 RHS, half of them: 657 us against
+    // 760 us with 8; rows of 1-7, 8 RHS: 1,170 against 1,010 us).  Two right-hand
+    // sides per lane halve the instructions and double what a lane waits for
+    // (FP64, 16 RHS: 3.44 against 4.66 ms on 47k rows per level, 1.35 against
+    // 1.57 ms on 5.9k, 753 against 683 us on 2.8k; FP32 turns earlier).
+    const long long entries = (long long)h->nnz - h->n, per_level = (long long)h->n / h->view[v].levels;
+    const bool long_rows = entries > 5LL * h->n && entries <= 8LL * h->n;
+    const bool pairs = cols >= 4 && per_level * cols >= (sizeof(T) == 8 ? 65536 : 32768);
+    // few elements per level: fewer warps, whose polls disturb each other less
+    // (FP64, 1,000 rows per level: 4 RHS 983 us with 8 warps, 1,028 with 12, 1,110
+    // with 16; 16 RHS 1,100, 1,009 and 1,050 us)
+    const int warps = per_level * cols < 12288 ? 8 : per_level * cols < 20480 ? 12 : 32;
+    CAPSP_CUDA(launch_stream_solve<T>(a, long_rows, pairs, warps, h->num_sms, st));
+    if (prof)
+        CAPSP_CUDA(cudaEventRecord(h->ev_k1, st));
+    return CAPSP_OK;
 }
 
 // chain kernel over view v, right-hand sides [0, nb) of b and x
@@ -1108,15 +1345,33 @@ static capsp_status_t enqueue_rows(capsp_handle_t h, int v, const T *b, T *x, in
                                    const Tuning &tn, cudaStream_t st)
 {
     const bool level = view_level(h, v);
-    const RowView &rv = h->view[v];
+    RowView &rv = h->view[v];
+    bool stream = false;
     if (level) {
         CAPSP_TRY(build_view(h, v));
-        CAPSP_TRY(ensure_xp(h, nrhs));
+        if (stream_wanted(h, v, tn, nrhs)) {
+            // a caller's capture that started before the layout was built goes
+            // on with the row kernels
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            const int cols = lanes_for_rhs(nrhs < 32 ? nrhs : 32);
+            if (!rv.stream.tried || (rv.stream.ok && rv.stream.pub_cap < cols))
+                CAPSP_CUDA(cudaStreamIsCapturing(st, &cs));
+            if (cs == cudaStreamCaptureStatusNone) {
+                CAPSP_TRY(ensure_stream(h, v, nrhs));
+                stream = rv.stream.ok;
+            }
+        }
+        if (!stream)
+            CAPSP_TRY(ensure_xp(h, nrhs));
     }
     for (int r0 = 0; r0 < nrhs; r0 += 32) {
         const int nb = nrhs - r0 < 32 ? nrhs - r0 : 32;
         if (chain_selected(h, v, tn, nrhs)) {
             CAPSP_TRY(enqueue_chain<T>(h, v, b + r0, x + r0, nb, ld, r0 == 0, st));
+            continue;
+        }
+        if (stream) {
+            CAPSP_TRY(enqueue_stream<T>(h, v, b + r0, x + r0, nb, ld, r0 == 0, st));
             continue;
         }
         int kind = tn.kind;
@@ -1374,12 +1629,16 @@ static capsp_status_t prepare(capsp_handle_t h, int nrhs, Op op)
         return ensure_column_scratch(h, nrhs);
     }
     const int v = view_of(h, op);
-    if (view_level(h, v)) {
+    if (view_level(h, v))
         CAPSP_TRY(build_view(h, v));
-        CAPSP_TRY(ensure_xp(h, nrhs));
-    }
     const Tuning tn = current_tuning(h, op, nrhs);
-    if ((tn.kind == kRowMix || tn.kind < 0) && !chain_selected(h, v, tn, nrhs)) {
+    if (view_level(h, v)) {
+        if (stream_wanted(h, v, tn, nrhs))
+            CAPSP_TRY(ensure_stream(h, v, nrhs));
+        CAPSP_TRY(ensure_xp(h, nrhs));  // fewer right-hand sides may go to the row kernels
+    }
+    if ((tn.kind == kRowMix || tn.kind < 0) && !chain_selected(h, v, tn, nrhs) &&
+        !stream_selected(h, v, tn, nrhs)) {
         MixTable *mt = nullptr;
         for (int r0 = 0; r0 < nrhs; r0 += 32) {
             const int nb = nrhs - r0 < 32 ? nrhs - r0 : 32;
@@ -1537,7 +1796,13 @@ extern "C" capsp_status_t capsp_solve_host(capsp_handle_t h, const void *b_host,
             (!column_driven(h, kOpSolve) && view_level(h, v) && !(wide_levels(h, v) && nrhs == 1))
                 ? pinned_alias(b_host, h->device)
                 : nullptr;
-        if (b_in_place) {
+        if (b_in_place && !chain_selected(h, v, tn, nrhs)) {
+            // the row kernels: many more rows wait for their b side by side
+            h->row_kernels_only = true;
+            const capsp_status_t sd = dispatch(h, kOpSolve, b_in_place, dx, nullptr, nullptr, nrhs, nrhs, st);
+            h->row_kernels_only = false;
+            CAPSP_TRY(sd);
+        } else if (b_in_place) {
             CAPSP_TRY(dispatch(h, kOpSolve, b_in_place, dx, nullptr, nullptr, nrhs, nrhs, st));
         } else {
             CAPSP_CUDA(cudaMemcpyAsync(db, b_host, bytes, cudaMemcpyHostToDevice, st));
@@ -1600,7 +1865,9 @@ extern "C" capsp_status_t capsp_solve_host(capsp_handle_t h, const void *b_host,
     h->seg_req = d_count;
     h->bready_req = b_flags ? d_bready : nullptr;
     h->seg_req_rows = seg_rows;
+    h->row_kernels_only = true;  // they wait for b's segments and count x's
     const capsp_status_t sd = dispatch(h, kOpSolve, db, dx, nullptr, nullptr, nrhs, nrhs, st);
+    h->row_kernels_only = false;
     h->seg_req = nullptr;
     h->bready_req = nullptr;
     if (side_upload)
@@ -1654,7 +1921,7 @@ extern "C" capsp_status_t capsp_autotune(capsp_handle_t h, const void *b, void *
         const bool allow_mix = alg == CAPSP_ALG_AUTO || alg == CAPSP_ALG_MIX;
         const int bpss[3] = {1, 2, 0};
         const Tuning base = untuned(h, kOpSolve);
-        if (chain_selected(h, v, base, nrhs))
+        if (chain_selected(h, v, base, nrhs) || stream_wanted(h, v, base, nrhs))
             cands.push_back(base);
         if (allow_thread) {
             // the default launch shape first: the search never ends worse
@@ -1865,8 +2132,8 @@ extern "C" capsp_status_t capsp_get_info(capsp_handle_t h, capsp_info_t *info)
             info->element_occupy = mit->second.eo;
             if (alg == CAPSP_ALG_AUTO)
                 alg = mit->second.wo > 0.0 ? CAPSP_ALG_MIX : CAPSP_ALG_WRTFST;
-        } else if (chain_selected(h, v, tn, 1)) {
-            // the chain kernel needs no selector table on the device; report
+        } else if (chain_selected(h, v, tn, 1) || stream_selected(h, v, tn, 1)) {
+            // these kernels need no selector table on the device; report
             // the row kernels' choice for this matrix
             std::vector<int> table((size_t)h->n + 2);
             info->mix_len = capsp_mix_table(h->n, h->view[v].h_lcum.data(), 0, 32, tn.border, table.data(),
@@ -1908,7 +2175,7 @@ extern "C" capsp_status_t capsp_hop_latency(int n, int stride, int dtype, float 
     const void *val = dtype == CAPSP_R_64F ? (const void *)v64.data() : (const void *)v32.data();
     capsp_handle_t h = nullptr;
     CAPSP_TRY(capsp_analyse(n, nnz, ptr.data(), idx.data(), val, dtype, CAPSP_FMT_CSR, CAPSP_LOWER, 0, &h));
-    h->chain = false;  // the probe measures the row kernel's hop
+    h->row_kernels_only = true;  // the probe measures the row kernel's hop
     const size_t vb = dtype == CAPSP_R_64F ? 8 : 4;
     void *d_b = nullptr, *d_x = nullptr;
     std::vector<double> ones64((size_t)n, 1.0);

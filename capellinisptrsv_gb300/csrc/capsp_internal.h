@@ -102,6 +102,25 @@ struct ChainArgs {
     int stuck_row;
 };
 
+// Arguments of the stream kernel (kernels_stream.cuh)
+template <typename T>
+struct StreamArgs {
+    const int2 *slice;  // first entry, entries of the longest row
+    long long npos;     // positions, 8 per slice
+    const int *row;     // row of every position (-1: none)
+    const T *linv;      // 1 / diagonal of every position
+    const int *idx;     // entry's position (-1: padding)
+    const T *val;       // entry's value, pre-scaled to -v / diagonal
+    T *xp;              // publication vector, all pending: lanes_for_rhs(nrhs) values per position
+    const T *b;
+    T *x;
+    long long ld;
+    int nrhs;           // <= 32
+    unsigned *words;    // three, zeroed before the launch
+    int *err;
+    WaitCfg wait;
+};
+
 // Arguments of the column-driven solve (SyncFree CSC kernel, and the
 // transpose solve that walks CSR rows as columns of the transpose).
 template <typename T>
@@ -157,6 +176,35 @@ inline bool row_hostio_supported(int kind, int rows_per_thread, int nrhs)
 template <typename T>
 cudaError_t launch_row_solve(const RowArgs<T> &a, int kind, int rows_per_thread, int block,
                              int blocks_per_sm, int num_sms, bool regcap, bool stage, cudaStream_t st);
+
+// Arrays of a stream layout being built or given new values, and the level layout
+// (view) it comes from
+template <typename T>
+struct StreamBuild {
+    const int2 *slice;
+    long long npos;
+    const int *pos;  // view position of a position (-1: none)
+    int *place;      // its inverse (building only)
+    const int *perm, *lptr, *lidx, *lsrc;
+    const T *lval, *view_linv;
+    int *row, *idx, *src;
+    T *val, *linv;
+};
+
+// one persistent block of up to `warps` warps per SM.  long_rows: rows of 9 to 12
+// entries are common; pairs: two right-hand sides per lane
+template <typename T>
+cudaError_t launch_stream_solve(const StreamArgs<T> &a, bool long_rows, bool pairs, int warps, int num_sms,
+                                cudaStream_t st);
+
+template <typename T>
+cudaError_t launch_stream_layout(const StreamBuild<T> &a, cudaStream_t st);
+
+// from the stored values; diag_src as for launch_level_values, whose results for
+// the view (view_linv, lval) it writes too
+template <typename T>
+cudaError_t launch_stream_values(const StreamBuild<T> &a, const int *diag_src, const T *stored, T *view_linv, T *lval,
+                                 int *bad, cudaStream_t st);
 
 // nrhs clusters: right-hand side r at b + r, x + r (row stride ld) and xp + r * n
 template <typename T>

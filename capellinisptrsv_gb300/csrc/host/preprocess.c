@@ -464,6 +464,64 @@ long long capsp_near_split(int n, const int *dep_ptr, const int *dep_idx, int gr
     return near_entries;
 }
 
+/* rows of a slice (kernels_stream.cuh) */
+#define CAPSP_SLICE_ROWS 8
+
+int capsp_stream_slices(int levels, const int *level_start)
+{
+    long long count = 0;
+    for (int l = 0; l < levels; ++l)
+        count += (level_start[l + 1] - level_start[l] + CAPSP_SLICE_ROWS - 1) / CAPSP_SLICE_ROWS;
+    return count <= 0x7fffffff / CAPSP_SLICE_ROWS ? (int)count : -1;
+}
+
+long long capsp_stream_layout(int levels, const int *level_start, const int *ptr, int diag, int *slice, int *pos)
+{
+    enum { W = CAPSP_SLICE_ROWS, TOP = 63 };
+    int *first = (int *)malloc(sizeof(int) * ((size_t)levels + 1));
+    if (!first)
+        return -1;
+    first[0] = 0;
+    for (int l = 0; l < levels; ++l)
+        first[l + 1] = first[l] + (level_start[l + 1] - level_start[l] + W - 1) / W;
+#pragma omp parallel for schedule(dynamic, 4)
+    for (int l = 0; l < levels; ++l) {
+        const int a = level_start[l], b = level_start[l + 1];
+        int by[TOP + 2];
+        memset(by, 0, sizeof(by));
+        for (int p = a; p < b; ++p) {
+            const int d = ptr[p + 1] - ptr[p] - diag;
+            by[TOP - (d < TOP ? d : TOP) + 1]++;
+        }
+        for (int t = 0; t <= TOP; ++t)
+            by[t + 1] += by[t];
+        int *out = pos + (size_t)W * first[l];
+        for (int p = a; p < b; ++p) {
+            const int d = ptr[p + 1] - ptr[p] - diag;
+            out[by[TOP - (d < TOP ? d : TOP)]++] = p;
+        }
+        for (int k = b - a; k < W * (first[l + 1] - first[l]); ++k)
+            out[k] = -1;
+        for (int k = first[l]; k < first[l + 1]; ++k) {
+            int m = 0;
+            for (int r = 0; r < W; ++r) {
+                const int p = pos[(size_t)W * k + r];
+                const int d = p < 0 ? 0 : ptr[p + 1] - ptr[p] - diag;
+                m = d > m ? d : m;
+            }
+            slice[2 * (size_t)k + 1] = m;
+        }
+    }
+    const int count = first[levels];
+    free(first);
+    long long at = 0;
+    for (int k = 0; k < count; ++k) {
+        slice[2 * (size_t)k] = (int)at;
+        at += (long long)W * slice[2 * (size_t)k + 1];
+    }
+    return at;
+}
+
 void capsp_indegree(int n, int nnz, const int *idx, int *indeg)
 {
     memset(indeg, 0, sizeof(int) * (size_t)(n > 0 ? n : 1));

@@ -561,6 +561,18 @@ def near_split(n, dep_ptr, dep_idx, span: int, group_rows: int = 32):
     return first, int(near)
 
 
+def stream_layout(level_start, dep_ptr):
+    """Slices of a level layout -> (slices as (first entry, longest row) pairs, pos of 8 per slice, entries)."""
+    level_start = np.ascontiguousarray(level_start, np.int32)
+    dep_ptr = np.ascontiguousarray(dep_ptr, np.int32)
+    levels = len(level_start) - 1
+    count = N.lib.capsp_stream_slices(levels, _ptr(level_start))
+    slices = np.empty((count, 2), np.int32)
+    pos = np.empty((count, 8), np.int32)
+    entries = N.lib.capsp_stream_layout(levels, _ptr(level_start), _ptr(dep_ptr), 0, _ptr(slices), _ptr(pos))
+    return slices, pos, int(entries)
+
+
 def transpose_structure(n, rowptr, colidx):
     """The structure transposed -> (tptr, tidx, src): new row j lists the stored
     rows holding index j, ascending; src maps new entries to stored ones."""

@@ -242,7 +242,7 @@ capsp_status_t capsp_grad_val(capsp_handle_t h, const void *y, const void *x,
 
 /* Backward of x = L^{-1} b: y = L^{-T} g (as capsp_solve_transpose), then
  * grad_val as capsp_grad_val; under CAPSP_ALG_SYNCFREE_CSC a CSR handle fuses
- * grad_val into its column-driven sweep.  No reference counterpart. */
+ * grad_val into its column-driven stream.  No reference counterpart. */
 capsp_status_t capsp_solve_transpose_grad(capsp_handle_t h, const void *g,
                                           const void *x, void *y, void *grad_val,
                                           int nrhs, int64_t ld, void *stream);
@@ -488,6 +488,18 @@ int capsp_level_layout(int n, const int *ptr, const int *idx, int upper, const i
  * Returns the number of near entries of all positions. */
 long long capsp_near_split(int n, const int *dep_ptr, const int *dep_idx, int group_rows, int span,
                            int *first_near);
+
+/* Slices of a level layout: the positions of each level, those of more
+ * dependencies first (ties in position order), 8 to a slice.  level_start
+ * (levels + 1 entries): first position of every level, and n; ptr (n + 1):
+ * position p has ptr[p+1] - ptr[p] - diag dependencies.
+ * capsp_stream_slices: how many there are (-1: too many for 32-bit positions).
+ * capsp_stream_layout: slice[2k] = first entry of slice k (wraps beyond 2^31),
+ * slice[2k+1] = m, the entries of its longest row (a slice holds 8 m entries);
+ * pos[8k + r] = position of the slice's row r (-1: none).  Returns the number of
+ * entries, or -1 when memory runs out. */
+int capsp_stream_slices(int levels, const int *level_start);
+long long capsp_stream_layout(int levels, const int *level_start, const int *ptr, int diag, int *slice, int *pos);
 
 /* In-degree analyser: histogram of idx (CUDA/SyncFree_csc/spts_syncfree_cuda2.h:10-21,
  * openCL/SynFree_csc/sptrsv_syncfree_serialref.h:6-23). */

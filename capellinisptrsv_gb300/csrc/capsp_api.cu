@@ -399,13 +399,19 @@ static capsp_status_t transpose_structure(int n, int nnz, const int *ptr, const 
 }
 
 // Rows per level up to which the chain kernel is the faster one, per wave of
-// right-hand sides (a cluster each, 16 of them resident).  Measured on GB300 in
+// right-hand sides (a cluster each; 15 are resident on a GB300).  Measured on GB300 in
 // FP64, chain against row kernel: 8 rows per level (1,048,576 Zipf rows) 28.3
 // against 100.9 ms, 13 (2,003 rows) 27 against 137 us, 115 (40,000 rows of 3-12
-// dependencies) 191 against 461 us, 200 (20,000 rows) 57 against 92 us, 377
-// (60,000 rows) 171 against 147 us.
+// dependencies) 162 against 460 us, 146 (38,261 rows of 3-10) 146 against 336 us,
+// 200 (20,000 rows of 1-5) 57 against 92 us, 377 (60,000 rows of 1-7) 171 against
+// 147 us.
 constexpr long long kChainLevelRows = 256;
-constexpr int kChainWave = 16;
+// Right-hand sides come in waves of as many clusters as are resident; from the
+// second wave on the row kernels, which take 16 at once, catch up sooner (16 RHS:
+// 40 rows per level 320 against 592 us, 114 rows 334 against 388 us, its
+// transpose 410 against 372 us).
+constexpr int kChainWave = 15;
+constexpr long long kChainWaveRows = 192;
 
 // Plan of the chain kernel for a level layout, and the first near entry of
 // every position.
@@ -415,14 +421,17 @@ constexpr int kChainWave = 16;
 // us with 8, 35 us with 16, 44 us with 4).  Wider levels are bound by the warps'
 // work per chunk and by the round trip that refills a slot: 16 warps (200 rows
 // per level: 93 us with 8, 73 us with 12, 60 us with 16) with four slots each
-// (54 us; three 62 us, two 82 us) while the near entries fit in slots that
-// small, else fewer slots.
+// (54 us; three 62 us, two 82 us), or fewer where the near entries of more than
+// one chunk in 32 would not fit in slots that small.  What does not fit goes back
+// to the feeders, oldest entries first; walked by the chain warps in global memory
+// it would cost tens of microseconds a chunk (40,000 rows of 3-12 dependencies,
+// transposed: 223 us when a few chunks did, 202 us now).
 //
-// The ring holds the whole solve where the slots leave room for that, else
-// 4,096 values for deep matrices and 8,192 for wider levels, whose dependencies
-// reach further back in positions.  Half of a ring that wraps is the reach of
-// near entries; the other half lets the chain warps drift apart and marks
-// positions pending ahead of them.
+// The ring holds the whole solve where it is short, else 4,096 values: less room
+// in the ring is more in the slots, and fewer entries are near (146 rows of 3-10
+// dependencies per level: 146 us, 236 us with 8,192).  Half of a ring that wraps is the reach of near
+// entries; the other half lets the chain warps drift apart and marks positions
+// pending ahead of them.
 static ChainPlan plan_chain(int n, int levels, size_t vb, const int *lptr, const int *lidx, std::vector<int> &lnear)
 {
     ChainPlan c;
@@ -433,38 +442,63 @@ static ChainPlan plan_chain(int n, int levels, size_t vb, const int *lptr, const
     while (c.ring < n && c.ring < (deep ? 16384 : 8192))
         c.ring *= 2;
     const bool all = c.ring >= n;
-    if (!all && deep)
+    if (!all)
         c.ring = 4096;
     const int span = all ? n : c.ring / 2;
     lnear.resize((size_t)n);
     const long long near_entries = capsp_near_split(n, lptr, lidx, 32, span, lnear.data());
-    const long long per_chunk = near_entries / ((n + 31) / 32);
     c.far = near_entries < (long long)lptr[n];
+    const int nchunks = (n + 31) / 32;
+    std::vector<int> chunk((size_t)nchunks);
+    for (int k = 0; k < nchunks; ++k)
+        for (int q = 32 * k; q < n && q < 32 * (k + 1); ++q)
+            chunk[(size_t)k] += lptr[q + 1] - lnear[(size_t)q];
     // the chain block holds words, ring and slots, a feeder words and a staging
     // area of a slot's size per warp
     const int words = 1024 + 32, hdr = 32 * (int)(vb + 8);
     const int shapes[4][2] = {{16, 4}, {16, 3}, {16, 2}, {8, 2}};  // warps, slots per warp
+    long long large = 0;
     for (int k = deep ? 3 : 0; k < 4; ++k) {
         c.warps = shapes[k][0];
         c.slots = c.warps * shapes[k][1];
         const int room = std::min((kChainSmem - words - c.ring * (int)vb) / c.slots, (kChainSmem - words) / kChainWarps);
         c.entries = (room - hdr) / (int)(vb + 2) / 8 * 8;
-        if (per_chunk + per_chunk / 4 <= c.entries)
+        large = std::count_if(chunk.begin(), chunk.end(), [&](int e) { return e > c.entries; });
+        if (32 * large <= nchunks)
             break;
+    }
+    // a chunk that does not fit has its oldest near entries folded by the feeder
+    // after all, as far as that goes
+    large = 0;
+    for (int k = 0; k < nchunks; ++k) {
+        const int q0 = 32 * k, q1 = std::min(n, q0 + 32);
+        for (int reach = span / 2; chunk[(size_t)k] > c.entries && reach >= 64; reach /= 2) {
+            chunk[(size_t)k] = 0;
+            for (int q = q0; q < q1; ++q) {
+                lnear[(size_t)q] = (int)(std::lower_bound(lidx + lnear[(size_t)q], lidx + lptr[q + 1], q0 - reach) - lidx);
+                chunk[(size_t)k] += lptr[q + 1] - lnear[(size_t)q];
+            }
+            c.far = true;
+        }
+        large += chunk[(size_t)k] > c.entries;
     }
     if (!all) {
         c.lag = (c.ring / 32 - span / 32 - 2) / 2;
         c.ahead = c.lag + 1;
     }
     // rows whose near entries do not fit are walked in global memory: fine for
-    // a few chunks, not for the average one
-    c.ok = per_chunk <= c.entries;
+    // some chunks (the first ones of a deep matrix, say), not for many
+    c.ok = near_entries / nchunks <= c.entries && 8 * large <= std::max(nchunks, 2048);
     return c;
 }
 
 // Rows per level from which the stream kernel is the faster one whatever the
 // number of right-hand sides (stream_wanted)
 constexpr long long kStreamAnyRows = 12288;
+// ... and the longest row it takes: a lane walks its row 8 or 12 entries at a
+// time, so longer ones are for the mixed row kernel's warps.  (Banded matrices
+// have some of 40 to 110 entries in their transposes, where few columns precede.)
+constexpr int kStreamLongest = 128;
 
 // Layout of the stream kernel for a view whose level layout is built
 // (rv.stream.ok, unless padding would double the entries); synchronous.
@@ -621,7 +655,7 @@ static capsp_status_t build_view(capsp_handle_t h, int v)
         return fail(CAPSP_ERR_CUDA, "level-schedule upload failed");
     if (bad != INT_MAX)
         return fail(CAPSP_ERR_INVALID, "zero or non-finite diagonal at schedule position %d", bad);
-    if (rv.longest <= 64 && (long long)n >= kStreamAnyRows * (long long)levels)
+    if (rv.longest <= kStreamLongest && (long long)n >= kStreamAnyRows * (long long)levels)
         return build_stream(h, rv);
     return CAPSP_OK;
 }
@@ -1203,7 +1237,7 @@ static bool chain_selected(capsp_handle_t h, int v, const Tuning &tn, int nrhs)
     const int waves = ((nrhs < 32 ? nrhs : 32) + kChainWave - 1) / kChainWave;
     return view_level(h, v) && rv.chain.ok && tn.kind < 0 && tn.dflt && !h->border_explicit && !h->row_kernels_only &&
            h->trace == nullptr && h->l2_mode == CAPSP_L2_HINTS &&
-           (long long)h->n * waves <= kChainLevelRows * (long long)rv.levels;
+           (long long)h->n * waves <= (waves > 1 ? kChainWaveRows : kChainLevelRows) * (long long)rv.levels;
 }
 
 // Whether a row-driven solve over view v would take the stream kernel (as above;
@@ -1225,7 +1259,7 @@ static bool stream_wanted(capsp_handle_t h, int v, const Tuning &tn, int nrhs)
     if (!view_level(h, v) || !rv.built || tn.kind >= 0 || !tn.dflt || h->border_explicit || h->trace != nullptr ||
         h->stuck_row >= 0 || h->l2_mode != CAPSP_L2_HINTS || h->row_kernels_only)
         return false;
-    if (rv.longest > 64)  // such rows want a warp (the mixed row kernel)
+    if (rv.longest > kStreamLongest)
         return false;
     const long long rows = (long long)h->n / rv.levels;  // per level
     const int cols = lanes_for_rhs(nrhs < 32 ? nrhs : 32);
@@ -1285,9 +1319,9 @@ static capsp_status_t enqueue_stream(capsp_handle_t h, int v, const T *b, T *x, 
     const bool long_rows = entries > 5LL * h->n && entries <= 8LL * h->n;
     const bool pairs = cols >= 4 && per_level * cols >= (sizeof(T) == 8 ? 65536 : 32768);
     // few elements per level: fewer warps, whose polls disturb each other less
-    // (FP64, 1,000 rows per level: 4 RHS 983 us with 8 warps, 1,028 with 12, 1,110
-    // with 16; 16 RHS 1,100, 1,009 and 1,050 us)
-    const int warps = per_level * cols < 12288 ? 8 : per_level * cols < 20480 ? 12 : 32;
+    // (FP64, 1,000 rows per level: 4 RHS 986 us with 8 warps, 1,028 with 12, 1,110
+    // with 16; 16 RHS 1,100, 1,004 and 1,050 us; 750 rows, 16 RHS: 513 and 433 us)
+    const int warps = per_level * cols < 10240 ? 8 : per_level * cols < 20480 ? 12 : 32;
     CAPSP_CUDA(launch_stream_solve<T>(a, long_rows, pairs, warps, h->num_sms, st));
     if (prof)
         CAPSP_CUDA(cudaEventRecord(h->ev_k1, st));

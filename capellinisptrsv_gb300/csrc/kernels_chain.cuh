@@ -467,23 +467,47 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
             // Every round loads, side by side, the ring value of the row's next
             // dependency, that entry's value and the next entry's index; a lane
             // that is done polls the word after the ring, which stays pending.
-            unsigned q0 = never;
+            // Single precision looks at two dependencies a round and folds the
+            // second too when both are there (200,000 Zipf rows: 4.18 -> 3.11 ms;
+            // in FP64 the second FMA holds up the lanes that have one: 131,072 rows
+            // of 40 dependencies 26 % slower).
+            constexpr bool two = sizeof(T) == 4;
+            unsigned q0 = never, q1 = never;
             unsigned at_v = slot_at + chain_header_bytes<T>() + (unsigned)sizeof(T) * (unsigned)k;
             unsigned at_i = slot_at + chain_header_bytes<T>() + (unsigned)sizeof(T) * (unsigned)a.entries + 2u * (unsigned)k;
             if (left > 0)
                 q0 = ring_at + (unsigned)sizeof(U) * shared_u16(at_i);
+            if (two && left > 1)
+                q1 = ring_at + (unsigned)sizeof(U) * shared_u16(at_i + 2u);
             while (__any_sync(kFullMask, left > 0)) {
 #pragma unroll
-                for (int t = 0; t < kChainRounds; ++t) {
-                    const U u = ring_load<T>(q0);
-                    const T v = VB::from(ring_load<T>(at_v));
-                    const unsigned next = shared_u16(at_i + 2u);
-                    if (!ring_pending(u)) {
-                        acc = fma(v, VB::from(u), acc);
-                        at_v += (unsigned)sizeof(T);
-                        at_i += 2u;
-                        q0 = ring_at + (unsigned)sizeof(U) * next;
-                        if (--left == 0) {
+                for (int t = 0; t < (two ? 4 : kChainRounds); ++t) {
+                    const U u0 = ring_load<T>(q0), u1 = two ? ring_load<T>(q1) : VB::kPending;
+                    const T v0 = VB::from(ring_load<T>(at_v));
+                    const T v1 = two ? VB::from(ring_load<T>(at_v + (unsigned)sizeof(T))) : T(0);
+                    const unsigned i1 = shared_u16(at_i + (two ? 4u : 2u));
+                    const unsigned i2 = two ? shared_u16(at_i + 6u) : 0u;
+                    if (!ring_pending(u0)) {
+                        acc = fma(v0, VB::from(u0), acc);
+                        int took = 1;
+                        if (two) {
+                            q0 = q1;
+                            q1 = ring_at + (unsigned)sizeof(U) * i1;
+                            if (!ring_pending(u1)) {
+                                acc = fma(v1, VB::from(u1), acc);
+                                q0 = q1;
+                                q1 = ring_at + (unsigned)sizeof(U) * i2;
+                                took = 2;
+                            }
+                        } else {
+                            q0 = ring_at + (unsigned)sizeof(U) * i1;
+                        }
+                        at_v += (unsigned)sizeof(T) * (unsigned)took;
+                        at_i += 2u * (unsigned)took;
+                        left -= took;
+                        if (two && left < 2)
+                            q1 = never;
+                        if (left == 0) {
                             ring_store(own, VB::to(acc));
                             q0 = never;
                         }
@@ -492,7 +516,7 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
                 if ((++polls & 255u) == 0u && left > 0 && sp.next(a.err, a.wait, row, (int)q0)) {
                     acc = VB::from(VB::kQNaN);
                     left = 0;
-                    q0 = never;
+                    q0 = q1 = never;
                     ring_store(own, VB::to(acc));
                 }
             }

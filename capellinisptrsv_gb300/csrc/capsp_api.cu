@@ -398,20 +398,18 @@ static capsp_status_t transpose_structure(int n, int nnz, const int *ptr, const 
     return CAPSP_OK;
 }
 
-// Rows per level up to which the chain kernel is the faster one, per wave of
-// right-hand sides (a cluster each; 15 are resident on a GB300).  Measured on GB300 in
-// FP64, chain against row kernel: 8 rows per level (1,048,576 Zipf rows) 28.3
-// against 100.9 ms, 13 (2,003 rows) 27 against 137 us, 115 (40,000 rows of 3-12
-// dependencies) 162 against 460 us, 146 (38,261 rows of 3-10) 146 against 336 us,
-// 200 (20,000 rows of 1-5) 57 against 92 us, 377 (60,000 rows of 1-7) 171 against
-// 147 us.
+// Rows per level up to which the chain kernel is the faster one.  Measured on
+// GB300 in FP64, chain against row kernel: 8 rows per level (1,048,576 Zipf rows)
+// 28.3 against 100.9 ms, 13 (2,003 rows) 27 against 137 us, 115 (40,000 rows of
+// 3-12 dependencies) 162 against 460 us, 146 (38,261 rows of 3-10) 146 against 336
+// us, 200 (20,000 rows of 1-5) 57 against 92 us, 377 (60,000 rows of 1-7) 171
+// against 147 us.
 constexpr long long kChainLevelRows = 256;
-// Right-hand sides come in waves of as many clusters as are resident; from the
-// second wave on the row kernels, which take 16 at once, catch up sooner (16 RHS:
-// 40 rows per level 320 against 592 us, 114 rows 334 against 388 us, its
-// transpose 410 against 372 us).
-constexpr int kChainWave = 15;
-constexpr long long kChainWaveRows = 192;
+// Right-hand sides up to which a cluster has five blocks (28 such clusters are
+// resident); above, four, which leaves a feeder warp for 48 slots.  Four blocks hold
+// a single right-hand side up by a tenth (20,000 rows in 100 levels: 65 us, 59 us),
+// but spare 32 of them a second turn (70 us, 120 us).
+constexpr int kChainWave = 28;
 
 // Plan of the chain kernel for a level layout, and the first near entry of
 // every position.
@@ -1231,13 +1229,11 @@ static capsp_status_t ensure_stream(capsp_handle_t h, int v, int nrhs)
 
 // whether a row-driven solve over view v takes the chain kernel: AUTO with the
 // default launch shape, outside the debug and L2-window modes
-static bool chain_selected(capsp_handle_t h, int v, const Tuning &tn, int nrhs)
+static bool chain_selected(capsp_handle_t h, int v, const Tuning &tn)
 {
     const RowView &rv = h->view[v];
-    const int waves = ((nrhs < 32 ? nrhs : 32) + kChainWave - 1) / kChainWave;
     return view_level(h, v) && rv.chain.ok && tn.kind < 0 && tn.dflt && !h->border_explicit && !h->row_kernels_only &&
-           h->trace == nullptr && h->l2_mode == CAPSP_L2_HINTS &&
-           (long long)h->n * waves <= (waves > 1 ? kChainWaveRows : kChainLevelRows) * (long long)rv.levels;
+           h->trace == nullptr && h->l2_mode == CAPSP_L2_HINTS;
 }
 
 // Whether a row-driven solve over view v would take the stream kernel (as above;
@@ -1356,7 +1352,8 @@ static capsp_status_t enqueue_chain(capsp_handle_t h, int v, const T *b, T *x, i
     a.nchunks = (h->n + 31) / 32;
     a.ring = cp.ring;
     a.warps = cp.warps;
-    a.slots = cp.slots;
+    a.blocks = nb <= kChainWave ? 5 : 4;
+    a.slots = std::min(cp.slots, (a.blocks - 1) * kChainWarps);
     a.entries = cp.entries;
     a.lag = cp.lag;
     a.ahead = cp.ahead;
@@ -1400,7 +1397,7 @@ static capsp_status_t enqueue_rows(capsp_handle_t h, int v, const T *b, T *x, in
     }
     for (int r0 = 0; r0 < nrhs; r0 += 32) {
         const int nb = nrhs - r0 < 32 ? nrhs - r0 : 32;
-        if (chain_selected(h, v, tn, nrhs)) {
+        if (chain_selected(h, v, tn)) {
             CAPSP_TRY(enqueue_chain<T>(h, v, b + r0, x + r0, nb, ld, r0 == 0, st));
             continue;
         }
@@ -1671,7 +1668,7 @@ static capsp_status_t prepare(capsp_handle_t h, int nrhs, Op op)
             CAPSP_TRY(ensure_stream(h, v, nrhs));
         CAPSP_TRY(ensure_xp(h, nrhs));  // fewer right-hand sides may go to the row kernels
     }
-    if ((tn.kind == kRowMix || tn.kind < 0) && !chain_selected(h, v, tn, nrhs) &&
+    if ((tn.kind == kRowMix || tn.kind < 0) && !chain_selected(h, v, tn) &&
         !stream_selected(h, v, tn, nrhs)) {
         MixTable *mt = nullptr;
         for (int r0 = 0; r0 < nrhs; r0 += 32) {
@@ -1811,7 +1808,7 @@ extern "C" capsp_status_t capsp_solve_host(capsp_handle_t h, const void *b_host,
     const int v = view_of(h, kOpSolve);
     const long long nseg_want = ((long long)h->n + kSegmentRowsMin - 1) / kSegmentRowsMin;
     const Tuning tn = current_tuning(h, kOpSolve, nrhs);
-    const bool progressive = !chain_selected(h, v, tn, nrhs) && !column_driven(h, kOpSolve) && view_level(h, v) && nseg_want >= 2 &&
+    const bool progressive = !chain_selected(h, v, tn) && !column_driven(h, kOpSolve) && view_level(h, v) && nseg_want >= 2 &&
                              row_hostio_supported(tn.kind < 0 ? kRowWrtFst : tn.kind, tn.R, nrhs) &&
                              wait_value32() != nullptr && pinned_alias(x_host, h->device) != nullptr;
     if (!progressive) {
@@ -1830,7 +1827,7 @@ extern "C" capsp_status_t capsp_solve_host(capsp_handle_t h, const void *b_host,
             (!column_driven(h, kOpSolve) && view_level(h, v) && !(wide_levels(h, v) && nrhs == 1))
                 ? pinned_alias(b_host, h->device)
                 : nullptr;
-        if (b_in_place && !chain_selected(h, v, tn, nrhs)) {
+        if (b_in_place && !chain_selected(h, v, tn)) {
             // the row kernels: many more rows wait for their b side by side
             h->row_kernels_only = true;
             const capsp_status_t sd = dispatch(h, kOpSolve, b_in_place, dx, nullptr, nullptr, nrhs, nrhs, st);
@@ -1955,7 +1952,7 @@ extern "C" capsp_status_t capsp_autotune(capsp_handle_t h, const void *b, void *
         const bool allow_mix = alg == CAPSP_ALG_AUTO || alg == CAPSP_ALG_MIX;
         const int bpss[3] = {1, 2, 0};
         const Tuning base = untuned(h, kOpSolve);
-        if (chain_selected(h, v, base, nrhs) || stream_wanted(h, v, base, nrhs))
+        if (chain_selected(h, v, base) || stream_wanted(h, v, base, nrhs))
             cands.push_back(base);
         if (allow_thread) {
             // the default launch shape first: the search never ends worse
@@ -2166,7 +2163,7 @@ extern "C" capsp_status_t capsp_get_info(capsp_handle_t h, capsp_info_t *info)
             info->element_occupy = mit->second.eo;
             if (alg == CAPSP_ALG_AUTO)
                 alg = mit->second.wo > 0.0 ? CAPSP_ALG_MIX : CAPSP_ALG_WRTFST;
-        } else if (chain_selected(h, v, tn, 1) || stream_selected(h, v, tn, 1)) {
+        } else if (chain_selected(h, v, tn) || stream_selected(h, v, tn, 1)) {
             // these kernels need no selector table on the device; report
             // the row kernels' choice for this matrix
             std::vector<int> table((size_t)h->n + 2);

@@ -66,9 +66,8 @@ struct RowArgs {
     const unsigned char *b_group_seg;
 };
 
-// The chain kernel (kernels_chain.cuh): a cluster of kChainBlocks blocks of
+// The chain kernel (kernels_chain.cuh): a cluster of ChainArgs::blocks blocks of
 // kChainWarps warps per right-hand side.
-constexpr int kChainBlocks = 8;
 constexpr int kChainWarps = 16;
 constexpr int kChainSmem = 232448;  // shared memory a block may take (227 KB)
 
@@ -91,8 +90,9 @@ struct ChainArgs {
     int n;
     int nchunks;  // of 32 positions
     int ring;     // values in the ring (a power of two)
+    int blocks;   // of a cluster: the chain block and the feeders
     int warps;    // warps of the chain block that take chunks
-    int slots;    // fed chunks in shared memory, a multiple of `warps`
+    int slots;    // fed chunks in shared memory, a multiple of `warps` and no more than the feeder warps
     int entries;  // near entries a slot holds (a multiple of 8)
     int lag;      // chunks that the warps may drift apart (0: the ring holds the whole solve)
     int ahead;    // chunks ahead of its own that a warp marks pending

@@ -35,7 +35,11 @@
 // another; chunks are fed and taken in schedule order, so the lowest
 // unfinished chunk can always proceed.  Every wait is bounded.
 //
-// Each right-hand side is solved by a cluster of its own.
+// Each right-hand side is solved by a cluster of its own, all of them at once:
+// 28 clusters of five blocks are resident on a GB300, and more right-hand sides
+// get four blocks each.  Five blocks have a feeder warp for each of the up to 64
+// slots, and more add nothing (8 blocks: 15 clusters resident, so that 16
+// right-hand sides took two turns: 20,000 rows in 493 levels 320 us, 166 us now).
 #pragma once
 
 #include "capsp_internal.h"
@@ -218,7 +222,7 @@ __device__ __forceinline__ void chain_feed(const ChainArgs<T> &a, unsigned base,
     typedef VBits<T> VB;
     typedef typename VB::U U;
     const int g = (rank - 1) * kChainWarps + warp;  // feeder number
-    const int per_slot = ((kChainBlocks - 1) * kChainWarps) / a.slots;
+    const int per_slot = ((a.blocks - 1) * kChainWarps) / a.slots;
     if (g >= per_slot * a.slots)
         return;
     const int s = g % a.slots;
@@ -544,7 +548,7 @@ template <typename T>
 __device__ __forceinline__ void chain_usher(const ChainArgs<T> &a, unsigned base, unsigned char *smem, int lane)
 {
     const volatile int *done = reinterpret_cast<const volatile int *>(smem + kChainDone);
-    const int per_slot = ((kChainBlocks - 1) * kChainWarps) / a.slots;
+    const int per_slot = ((a.blocks - 1) * kChainWarps) / a.slots;
     int c = lane < a.warps ? lane : a.nchunks;  // the chain warp's chunk to hand back next
     RoleWait rw;
     while (__any_sync(kFullMask, c < a.nchunks)) {
@@ -567,8 +571,7 @@ __device__ __forceinline__ void chain_usher(const ChainArgs<T> &a, unsigned base
 }
 
 template <typename T>
-__global__ void __cluster_dims__(kChainBlocks, 1, 1) __launch_bounds__(kChainThreads, 1)
-    chain_solve_kernel(const ChainArgs<T> a)
+__global__ void __launch_bounds__(kChainThreads, 1) chain_solve_kernel(const ChainArgs<T> a)
 {
     typedef VBits<T> VB;
     typedef typename VB::U U;
@@ -576,7 +579,7 @@ __global__ void __cluster_dims__(kChainBlocks, 1, 1) __launch_bounds__(kChainThr
     const unsigned base = (unsigned)__cvta_generic_to_shared(chain_smem);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rank = (int)cluster_ctarank();
-    const int rhs = (int)(blockIdx.x / kChainBlocks);
+    const int rhs = (int)(blockIdx.x / (unsigned)a.blocks);
     if (rank == 0) {
         if (threadIdx.x < (unsigned)a.slots)
             mbar_init(base + kChainFull + 8u * threadIdx.x, 1u);
@@ -614,8 +617,18 @@ cudaError_t launch_chain_solve(const ChainArgs<T> &a, int nrhs, cudaStream_t st)
     cudaError_t e = cudaFuncSetAttribute(chain_solve_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess)
         return e;
-    chain_solve_kernel<T><<<(unsigned)(nrhs * kChainBlocks), kChainThreads, smem, st>>>(a);
-    return cudaGetLastError();
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)a.blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nrhs * a.blocks));
+    cfg.blockDim = dim3(kChainThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, chain_solve_kernel<T>, a);
 }
 
 }  // namespace capsp

@@ -129,3 +129,18 @@ def test_chain_timeout_is_reported(name):
     s.debug_stuck_row(-1, timeout_s=10.0)
     assert rel_inf_err(host(s.solve(dev(b))), xo) <= 1e-12
     s.status()
+
+
+@pytest.mark.parametrize("k", [28, 29, 32, 61])
+@pytest.mark.parametrize("name", ["n33", "wrap_near", "wrap_far", "deep_far_heavy"])
+def test_chain_clusters_of_five_and_four_blocks(name, k):
+    """Each right-hand side comes out as when it is solved alone, bit for bit, on
+    either side of the line between the cluster sizes and with a remainder."""
+    m = MATRICES[name]()
+    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(m.val))
+    b = np.random.default_rng(k).standard_normal((m.n, k))
+    x = host(s.solve(dev(b)))
+    for r in (0, 27, k - 1):
+        alone = host(s.solve(dev(b[:, r])))
+        assert np.array_equal(x[:, r].view(np.uint64), alone.view(np.uint64)), r
+    s.status()

@@ -400,8 +400,12 @@ def run_native(args):
     alg_bytes = algorithmic_bytes(m.n, m.nnz, s_bytes)
     peak, peak_kind = peaks()
     achieved = alg_bytes / (kms * 1e-3) / 1e9
-    traffic = profile_traffic("row_solve", args.workload + "_" + args.dtype)
     info = solver.info()
+    # "auto" solves levels of up to 256 rows with the chain kernel: one launch, and a
+    # fill where dependencies reach beyond its ring (not counted in gpu_launches)
+    chain = m.n <= 256 * info["levels"]
+    kernel = "chain_solve" if chain else "row_solve"
+    traffic = profile_traffic(kernel, args.workload + "_" + args.dtype)
     # dependency-chain floor: a solve of L levels takes at least L - 1 hops,
     # each costing at least one publication's detection on another warp
     hop_ns = cs.hop_latency(n=262_144, stride=64, dtype=dt)
@@ -427,7 +431,7 @@ def run_native(args):
                        "parallelism": f"replicas x{world}" if world > 1 else "single GPU"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                         "kernel": "row_solve_kernel", "kernel_ms": kms,
+                         "kernel": kernel + "_kernel", "kernel_ms": kms,
                          "algorithmic_bytes_per_launch": alg_bytes,
                          "hop_ns": hop_ns, "latency_floor_ms": floor_ms,
                          "frac_of_floor": floor_ms / kms if kms > 0 else None,
@@ -437,7 +441,7 @@ def run_native(args):
             "cpu_baseline": cpu,
             "e2e": e2e,
             "cusparse_spsv": vendor,
-            "gpu_launches": 2 * args.steps,
+            "gpu_launches": (1 if chain else 2) * args.steps,
             "gflops_2nnz": world * 2.0 * m.nnz / (ms * 1e-3) / 1e9,
             "gbs_algorithmic": alg_bytes / (ms * 1e-3) / 1e9,
             "rel_err_vs_cpu_reference": rel, "max_abs_x_minus_ones": max_dev,
@@ -721,10 +725,12 @@ def measure_batched(args, ks, cpu_seconds, e2e: bool = True):
         entry["speedup_vs_loop"] = entry["solves_per_s"] / entry["loop_solves_per_s"]
         alg = algorithmic_bytes(m.n, m.nnz, 8, k)
         # DRAM bytes per launch from a committed capture of this k (default batch)
-        traffic = profile_traffic("row_solve", f"batched_k{k}_f64") if nsys == BATCH_NSYS else None
+        # (the stream kernel, unless the autotuner preferred a launch shape of the row kernel)
+        kernel = "stream_solve" if info["blocks_per_sm"] == 0 else "row_solve"
+        traffic = profile_traffic(kernel, f"batched_k{k}_f64") if nsys == BATCH_NSYS else None
         entry["roofline"] = {"bound": "hbm", "achieved": alg / (kms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                              "frac": alg / (kms * 1e-3) / 1e9 / peak, "traffic": traffic, "peak_kind": peak_kind,
-                             "kernel": "row_solve_kernel", "kernel_ms": kms, "algorithmic_bytes_per_launch": alg}
+                             "kernel": kernel + "_kernel", "kernel_ms": kms, "algorithmic_bytes_per_launch": alg}
         sweep.append(entry)
         del b_d, x_d, cols, calls
 
@@ -912,14 +918,15 @@ def measure_autograd(args, cpu_seconds):
     peak, peak_kind = peaks()
     fwd_bytes = algorithmic_bytes(n, m.nnz, 8, k)
     grad_bytes = _grad_bytes(n, m.nnz, 8, k)
+    solve = "stream_solve" if k >= 4 else "row_solve"  # the kernel that "auto" takes
     kernels = {
-        "forward_row_solve": {"kernel": "row_solve_kernel", "kernel_ms": kf, "algorithmic_bytes_per_launch": fwd_bytes,
+        "forward_row_solve": {"kernel": solve + "_kernel", "kernel_ms": kf, "algorithmic_bytes_per_launch": fwd_bytes,
                               "achieved": fwd_bytes / (kf * 1e-3) / 1e9,
-                              "traffic": profile_traffic("row_solve", f"grad_1m_{k}rhs_f64")},
-        "transpose_row_solve": {"kernel": "row_solve_kernel over the transposed view", "kernel_ms": kt,
+                              "traffic": profile_traffic(solve, f"grad_1m_{k}rhs_f64")},
+        "transpose_row_solve": {"kernel": solve + "_kernel over the transposed view", "kernel_ms": kt,
                                 "algorithmic_bytes_per_launch": fwd_bytes,
                                 "achieved": fwd_bytes / (kt * 1e-3) / 1e9,
-                                "traffic": profile_traffic("row_solve_transpose", f"grad_1m_{k}rhs_f64")},
+                                "traffic": profile_traffic(solve + "_transpose", f"grad_1m_{k}rhs_f64")},
         "grad_val": {"kernel": "grad_val_kernel", "kernel_ms": kg, "algorithmic_bytes_per_launch": grad_bytes,
                      "achieved": grad_bytes / (kg * 1e-3) / 1e9,
                      "fp64_fma_per_launch": float(m.nnz) * k,

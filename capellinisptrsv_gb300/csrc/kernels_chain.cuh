@@ -23,8 +23,8 @@
 // diverge 300), and a row's dependencies that land together cost a round each.
 // 1,048,576 Zipf rows in 126k levels: 100.9 ms with the row kernel (0.79 us per
 // level), 28.3 ms here (0.22 us); 131,072 rows of 40 dependencies in 87k
-// levels: 64.7 -> 11.5 ms; 2,003 rows in 153 levels: 137 -> 27 us (one launch
-// instead of two); 20,000 rows in 100 levels: 92 -> 57 us.
+// levels: 64.7 -> 10.7 ms; 2,003 rows in 153 levels: 137 -> 27 us (one launch
+// instead of two); 20,000 rows in 100 levels: 92 -> 56 us.
 //
 // Per round a lane loads its next dependency's ring value together with that
 // entry's value and the next entry's index, instead of carrying entries in
@@ -214,6 +214,24 @@ __device__ __forceinline__ T chain_far_value(const ChainArgs<T> &a, const typena
     return VB::from(u);
 }
 
+// acc + v * u.  A lane sums its row's entries one after the other; in single
+// precision what rounding drops on the way is summed beside it and added at the
+// end, off the chain (60,000 Zipf rows of 40 and more dependencies, 2-norm against 64
+// bits: 5.0e-8, plainly 1.6e-7, the row kernel's tree of 32 lanes 3.7e-8).
+__device__ __forceinline__ double chain_fold(double v, double u, double acc, double &) { return fma(v, u, acc); }
+__device__ __forceinline__ float chain_fold(float v, float u, float acc, float &low)
+{
+    const float sum = fmaf(v, u, acc);
+    low += fmaf(v, u, acc - sum);
+    return sum;
+}
+__device__ __forceinline__ double chain_sum(double acc, double) { return acc; }
+__device__ __forceinline__ float chain_sum(float acc, float low)
+{
+    const float sum = acc + low;
+    return sum == sum ? sum : acc;  // an infinite sum has no remainder (infinity - infinity)
+}
+
 // Feeder: chunks c = s, s + step, ... of one slot.
 template <typename T>
 __device__ __forceinline__ void chain_feed(const ChainArgs<T> &a, unsigned base, unsigned char *smem, int rank,
@@ -247,7 +265,7 @@ __device__ __forceinline__ void chain_feed(const ChainArgs<T> &a, unsigned base,
         const int p = (int)(32 * c) + lane;
         const bool act = p < a.n;
         int row = 0, fs = 0, ns = 0, ne = 0;
-        T acc = T(0);
+        T acc = T(0), low = T(0);
         if (act) {
             row = ld_stream(a.perm + p, stream);
             fs = ld_stream(a.lptr + p, stream);
@@ -315,8 +333,9 @@ __device__ __forceinline__ void chain_feed(const ChainArgs<T> &a, unsigned base,
 #pragma unroll
             for (int t = 0; t < 8; ++t)
                 if (k + t < fe)
-                    acc = fma(v[t], chain_far_value<T>(a, xp, q[t], u[t], p, keep), acc);
+                    acc = chain_fold(v[t], chain_far_value<T>(a, xp, q[t], u[t], p, keep), acc, low);
         }
+        acc = chain_sum(acc, low);
         // ... of heavy rows: all lanes on one row, then a butterfly sum
         __syncwarp();
         for (unsigned m = __ballot_sync(kFullMask, heavy); m != 0u; m &= m - 1u) {
@@ -416,7 +435,7 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
         const T *s_val = reinterpret_cast<const T *>(slot + chain_header_bytes<T>());
         const unsigned short *s_idx = reinterpret_cast<const unsigned short *>(s_val + a.entries);
         bool open = p < a.n;
-        T acc = reinterpret_cast<const T *>(slot)[lane];
+        T acc = reinterpret_cast<const T *>(slot)[lane], low = T(0);
         const int row = reinterpret_cast<const int *>(slot + 32 * sizeof(T))[lane];
         const unsigned meta = reinterpret_cast<const unsigned *>(slot + 32 * sizeof(T) + 128)[lane];
         int k = (int)(meta & 0xffffu), left = open && meta != kChainSpill ? (int)(meta >> 16) : 0;
@@ -445,7 +464,7 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
                         const T v = glob ? ld_stream(a.lval + j0, stream) : left > 0 ? s_val[k] : T(0);
                         const U u = ring_load<T>(ring_at + (unsigned)sizeof(U) * q);
                         if (!ring_pending(u)) {
-                            acc = fma(v, VB::from(u), acc);
+                            acc = chain_fold(v, VB::from(u), acc, low);
                             if (glob) {
                                 ++j0;
                             } else {
@@ -460,6 +479,7 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
                         }
                     }
                     if (j0 >= j1 && left == 0 && !wait_own) {
+                        acc = chain_sum(acc, low);
                         ring_store(own, VB::to(acc));
                         open = false;
                     }
@@ -472,7 +492,7 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
             // dependency, that entry's value and the next entry's index; a lane
             // that is done polls the word after the ring, which stays pending.
             // Single precision looks at two dependencies a round and folds the
-            // second too when both are there (200,000 Zipf rows: 4.18 -> 3.11 ms;
+            // second too when both are there (200,000 Zipf rows: 4.18 -> 3.40 ms;
             // in FP64 the second FMA holds up the lanes that have one: 131,072 rows
             // of 40 dependencies 26 % slower).
             constexpr bool two = sizeof(T) == 4;
@@ -492,13 +512,13 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
                     const unsigned i1 = shared_u16(at_i + (two ? 4u : 2u));
                     const unsigned i2 = two ? shared_u16(at_i + 6u) : 0u;
                     if (!ring_pending(u0)) {
-                        acc = fma(v0, VB::from(u0), acc);
+                        acc = chain_fold(v0, VB::from(u0), acc, low);
                         int took = 1;
                         if (two) {
                             q0 = q1;
                             q1 = ring_at + (unsigned)sizeof(U) * i1;
                             if (!ring_pending(u1)) {
-                                acc = fma(v1, VB::from(u1), acc);
+                                acc = chain_fold(v1, VB::from(u1), acc, low);
                                 q0 = q1;
                                 q1 = ring_at + (unsigned)sizeof(U) * i2;
                                 took = 2;
@@ -512,6 +532,7 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
                         if (two && left < 2)
                             q1 = never;
                         if (left == 0) {
+                            acc = chain_sum(acc, low);
                             ring_store(own, VB::to(acc));
                             q0 = never;
                         }

@@ -165,3 +165,24 @@ def test_stream_beside_other_work():
     for s, x in zip(solvers, outs):
         s.status()
         assert rel_inf_err(host(x), xo) <= 1e-12
+
+
+def test_row_kernel_first_runs_inside_a_capture_after_stream_solves():
+    """The scratch that warm-up solves in the stream kernel did not need is
+    allocated without breaking the caller's capture."""
+    m = cs.generate(n=60_000, kmin=1, kmax=5, band=30_000, seed=21)
+    b = np.random.default_rng(21).standard_normal((m.n, 8)).astype(np.float32)
+    v = m.val.astype(np.float32)
+    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(v))
+    bd = dev(b)
+    x = torch.empty_like(bd)
+    s.solve(bd, x)
+    s.set_algorithm("wrtfst")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        s.solve(bd, x)
+    x.zero_()
+    g.replay()
+    assert rel_inf_err(host(x), oracle.solve_csr_lower(m.rowptr, m.colidx, v, b)) <= 1e-5
+    s.status()

@@ -402,7 +402,7 @@ def run_native(args):
     achieved = alg_bytes / (kms * 1e-3) / 1e9
     info = solver.info()
     # "auto" solves levels of up to 256 rows with the chain kernel: one launch, and a
-    # fill where dependencies reach beyond its ring (not counted in gpu_launches)
+    # fill where dependencies of a long solve reach beyond its ring (not counted in gpu_launches)
     chain = m.n <= 256 * info["levels"]
     kernel = "chain_solve" if chain else "row_solve"
     traffic = profile_traffic(kernel, args.workload + "_" + args.dtype)

@@ -96,6 +96,7 @@ struct ChainArgs {
     int entries;  // near entries a slot holds (a multiple of 8)
     int lag;      // chunks that the warps may drift apart (0: the ring holds the whole solve)
     int ahead;    // chunks ahead of its own that a warp marks pending
+    int fill;     // mark the publication vector pending before the solve
     int reset_err;
     int *err;
     WaitCfg wait;

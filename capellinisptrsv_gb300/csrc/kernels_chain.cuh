@@ -24,7 +24,7 @@
 // 1,048,576 Zipf rows in 126k levels: 100.9 ms with the row kernel (0.79 us per
 // level), 28.3 ms here (0.22 us); 131,072 rows of 40 dependencies in 87k
 // levels: 64.7 -> 10.7 ms; 2,003 rows in 153 levels: 137 -> 27 us (one launch
-// instead of two); 20,000 rows in 100 levels: 92 -> 56 us.
+// instead of two); 20,000 rows in 100 levels: 92 -> 53 us.
 //
 // Per round a lane loads its next dependency's ring value together with that
 // entry's value and the next entry's index, instead of carrying entries in
@@ -615,8 +615,14 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_solve_kernel(const Cha
     } else if (threadIdx.x < kChainWarps) {
         reinterpret_cast<volatile unsigned *>(chain_smem + kChainFreed)[threadIdx.x] = 0u;
     }
-    cluster_sync_all();
     T *xp = a.xp != nullptr ? a.xp + (size_t)rhs * (size_t)a.n : nullptr;
+    if (a.fill) {
+        // only this cluster polls and publishes here, after its barrier
+        const unsigned long long keep = l2_policy_evict_last();
+        for (int k = rank * kChainThreads + (int)threadIdx.x; k < a.n; k += a.blocks * kChainThreads)
+            st_relaxed(reinterpret_cast<U *>(xp) + k, VB::kPending, keep);
+    }
+    cluster_sync_all();
     if (rank != 0) {
         if (warp < kChainWarps)
             chain_feed<T>(a, base, chain_smem, rank, warp, lane, a.b + rhs, xp);

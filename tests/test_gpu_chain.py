@@ -144,3 +144,16 @@ def test_chain_clusters_of_five_and_four_blocks(name, k):
         alone = host(s.solve(dev(b[:, r])))
         assert np.array_equal(x[:, r].view(np.uint64), alone.view(np.uint64)), r
     s.status()
+
+
+@pytest.mark.parametrize("n", [131_072, 131_073])
+def test_chain_marks_short_vectors_pending_itself(n):
+    """Either side of the length up to which the kernel fills the publication
+    vector; the second solve would read the first one's values where it did not."""
+    m = cs.generate("zipf40_1m", n=n, seed=12)
+    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(m.val))
+    for seed in (1, 2):
+        b = cs.normal(m.n, seed=seed)
+        x = host(s.solve(dev(b)))
+        assert rel_inf_err(x, oracle.solve_csr_lower(m.rowptr, m.colidx, m.val, b)) <= 1e-12
+    s.status()

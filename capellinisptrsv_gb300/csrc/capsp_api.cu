@@ -5,6 +5,7 @@
 #include "capsp.h"
 #include "capsp_internal.h"
 #include "graph_cache.h"
+#include "route.h"
 
 #include <algorithm>
 #include <atomic>
@@ -398,13 +399,6 @@ static capsp_status_t transpose_structure(int n, int nnz, const int *ptr, const 
     return CAPSP_OK;
 }
 
-// Rows per level up to which the chain kernel is the faster one.  Measured on
-// GB300 in FP64, chain against row kernel: 8 rows per level (1,048,576 Zipf rows)
-// 28.3 against 100.9 ms, 13 (2,003 rows) 27 against 137 us, 115 (40,000 rows of
-// 3-12 dependencies) 162 against 460 us, 146 (38,261 rows of 3-10) 146 against 336
-// us, 200 (20,000 rows of 1-5) 57 against 92 us, 377 (60,000 rows of 1-7) 171
-// against 147 us.
-constexpr long long kChainLevelRows = 256;
 // Right-hand sides up to which a cluster has five blocks (28 such clusters are
 // resident); above, four, which leaves a feeder warp for 48 slots.  Four blocks hold
 // a single right-hand side up by a tenth (20,000 rows in 100 levels: 65 us, 59 us),
@@ -439,7 +433,7 @@ constexpr int kChainFill = 131072;
 static ChainPlan plan_chain(int n, int levels, size_t vb, const int *lptr, const int *lidx, std::vector<int> &lnear)
 {
     ChainPlan c;
-    if ((long long)n > kChainLevelRows * (long long)levels)
+    if (!chain_levels(n, levels))
         return c;
     const bool deep = (long long)n < 64LL * (long long)levels;
     c.ring = 1024;
@@ -495,14 +489,6 @@ static ChainPlan plan_chain(int n, int levels, size_t vb, const int *lptr, const
     c.ok = near_entries / nchunks <= c.entries && 8 * large <= std::max(nchunks, 2048);
     return c;
 }
-
-// Rows per level from which the stream kernel is the faster one whatever the
-// number of right-hand sides (stream_wanted)
-constexpr long long kStreamAnyRows = 12288;
-// ... and the longest row it takes: a lane walks its row 8 or 12 entries at a
-// time, so longer ones are for the mixed row kernel's warps.  (Banded matrices
-// have some of 40 to 110 entries in their transposes, where few columns precede.)
-constexpr int kStreamLongest = 128;
 
 // Layout of the stream kernel for a view whose level layout is built
 // (rv.stream.ok, unless padding would double the entries); synchronous.
@@ -1271,55 +1257,32 @@ static capsp_status_t ensure_stream(capsp_handle_t h, int v, int nrhs)
     return CAPSP_OK;
 }
 
-// whether a row-driven solve over view v takes the chain kernel: AUTO with the
-// default launch shape, outside the debug and L2-window modes
-static bool chain_selected(capsp_handle_t h, int v, const Tuning &tn)
+// The kernel that a row-driven solve over view v, whose level layout is built, asks
+// for (auto_kernel): AUTO with the default launch shape, outside the debug and
+// L2-window modes; the debug hook of a row that never publishes keeps a solve that
+// the stream kernel would take on the row kernels.
+static SolveKernel kernel_wanted(capsp_handle_t h, int v, const Tuning &tn, int nrhs)
 {
     const RowView &rv = h->view[v];
-    return view_level(h, v) && rv.chain.ok && tn.kind < 0 && tn.dflt && !h->border_explicit && !h->row_kernels_only &&
-           h->trace == nullptr && h->l2_mode == CAPSP_L2_HINTS;
+    if (!view_level(h, v) || !rv.built || tn.kind >= 0 || !tn.dflt || h->border_explicit || h->row_kernels_only ||
+        h->trace != nullptr || h->l2_mode != CAPSP_L2_HINTS)
+        return kSolveRows;
+    ViewShape s;
+    s.n = h->n;
+    s.levels = rv.levels;
+    s.entries = (long long)h->nnz - h->n;
+    s.longest = rv.longest;
+    s.chain = rv.chain.ok;
+    s.f64 = h->dtype == CAPSP_R_64F;
+    const SolveKernel k = auto_kernel(s, lanes_for_rhs(nrhs < 32 ? nrhs : 32));
+    return k == kSolveStream && h->stuck_row >= 0 ? kSolveRows : k;
 }
 
-// Whether a row-driven solve over view v would take the stream kernel (as above;
-// the debug hook of a row that never publishes stays with the row kernels).
-// The row kernels follow a chain of dependencies faster, the stream kernel gets
-// through more rows.  Measured on GB300, time of the row kernel / time of the
-// stream kernel:
-//   1 RHS: FP64 0.87 at 5.9k rows per level, 1.03 at 12k, 1.25 at 14k, 1.36 at 47k;
-//          FP32 0.92, -, 1.40, 1.42
-//   2 RHS: FP64 0.91 at 5.9k, 1.47 at 14k, 1.74 at 47k; FP32 1.00, 1.51, 1.86
-//   4 and more, FP32: 1.04 to 3.0 from 700 rows per level on
-//   4 and more, FP64: by the rows' length.  5 to 8 entries on average (12 fit a
-//          lane, 8 a lane of the row kernel): 1.05 to 1.24 from 700 rows per level
-//          on.  Shorter: 1.03 at 4.6k row-columns per level, 0.96 at 11k, 1.17 at
-//          23k, 1.10 to 1.49 above.  Longer: 0.94 at 6k, 1.10 at 12k.
-static bool stream_wanted(capsp_handle_t h, int v, const Tuning &tn, int nrhs)
+// ... and the one it runs in, as far as the stream layout has been built
+static SolveKernel kernel_ready(capsp_handle_t h, int v, const Tuning &tn, int nrhs)
 {
-    const RowView &rv = h->view[v];
-    if (!view_level(h, v) || !rv.built || tn.kind >= 0 || !tn.dflt || h->border_explicit || h->trace != nullptr ||
-        h->stuck_row >= 0 || h->l2_mode != CAPSP_L2_HINTS || h->row_kernels_only)
-        return false;
-    if (rv.longest > kStreamLongest)
-        return false;
-    const long long rows = (long long)h->n / rv.levels;  // per level
-    const int cols = lanes_for_rhs(nrhs < 32 ? nrhs : 32);
-    if (rows >= kStreamAnyRows)
-        return true;
-    if (rows < kChainLevelRows || cols == 1)
-        return false;
-    if (cols == 2)
-        return rows >= 8192;
-    if (h->dtype == CAPSP_R_32F)
-        return true;
-    const long long entries = (long long)h->nnz - h->n;
-    if (entries > 8LL * h->n)
-        return rows * cols >= 10240;
-    return entries > 5LL * h->n || rows * cols >= 16384;
-}
-
-static bool stream_selected(capsp_handle_t h, int v, const Tuning &tn, int nrhs)
-{
-    return h->view[v].stream.ok && stream_wanted(h, v, tn, nrhs);
+    const SolveKernel k = kernel_wanted(h, v, tn, nrhs);
+    return k == kSolveStream && !h->view[v].stream.ok ? kSolveRows : k;
 }
 
 // stream kernel over view v, right-hand sides [0, nb) of b and x
@@ -1375,6 +1338,8 @@ static capsp_status_t enqueue_chain(capsp_handle_t h, int v, const T *b, T *x, i
 {
     const RowView &rv = h->view[v];
     const ChainPlan &cp = rv.chain;
+    if (cp.far && h->xp_cap < nb)
+        return fail(CAPSP_ERR_CUDA, "publication vector of %d right-hand sides, %d are solved", h->xp_cap, nb);
     // far dependencies are polled in the publication vector, which starts
     // all-pending: a single right-hand side marks a short one itself, and needs
     // one launch, as it does without far dependencies
@@ -1424,31 +1389,33 @@ static capsp_status_t enqueue_rows(capsp_handle_t h, int v, const T *b, T *x, in
 {
     const bool level = view_level(h, v);
     RowView &rv = h->view[v];
-    bool stream = false;
+    // decided once: the scratch below is that of the kernel that runs
+    SolveKernel kernel = kSolveRows;
     if (level) {
         CAPSP_TRY(build_view(h, v));
-        if (stream_wanted(h, v, tn, nrhs)) {
+        kernel = kernel_wanted(h, v, tn, nrhs);
+        if (kernel == kSolveStream) {
             // a caller's capture that started before the layout was built goes
             // on with the row kernels
             cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
             const int cols = lanes_for_rhs(nrhs < 32 ? nrhs : 32);
             if (!rv.stream.tried || (rv.stream.ok && rv.stream.pub_cap < cols))
                 CAPSP_CUDA(cudaStreamIsCapturing(st, &cs));
-            if (cs == cudaStreamCaptureStatusNone) {
+            if (cs == cudaStreamCaptureStatusNone)
                 CAPSP_TRY(ensure_stream(h, v, nrhs));
-                stream = rv.stream.ok;
-            }
+            if (cs != cudaStreamCaptureStatusNone || !rv.stream.ok)
+                kernel = kSolveRows;
         }
-        if (!stream)
+        if (kernel != kSolveStream)
             CAPSP_TRY(ensure_xp(h, nrhs));
     }
     for (int r0 = 0; r0 < nrhs; r0 += 32) {
         const int nb = nrhs - r0 < 32 ? nrhs - r0 : 32;
-        if (chain_selected(h, v, tn)) {
+        if (kernel == kSolveChain) {
             CAPSP_TRY(enqueue_chain<T>(h, v, b + r0, x + r0, nb, ld, r0 == 0, st));
             continue;
         }
-        if (stream) {
+        if (kernel == kSolveStream) {
             CAPSP_TRY(enqueue_stream<T>(h, v, b + r0, x + r0, nb, ld, r0 == 0, st));
             continue;
         }
@@ -1711,12 +1678,11 @@ static capsp_status_t prepare(capsp_handle_t h, int nrhs, Op op)
         CAPSP_TRY(build_view(h, v));
     const Tuning tn = current_tuning(h, op, nrhs);
     if (view_level(h, v)) {
-        if (stream_wanted(h, v, tn, nrhs))
+        if (kernel_wanted(h, v, tn, nrhs) == kSolveStream)
             CAPSP_TRY(ensure_stream(h, v, nrhs));
         CAPSP_TRY(ensure_xp(h, nrhs));  // fewer right-hand sides may go to the row kernels
     }
-    if ((tn.kind == kRowMix || tn.kind < 0) && !chain_selected(h, v, tn) &&
-        !stream_selected(h, v, tn, nrhs)) {
+    if ((tn.kind == kRowMix || tn.kind < 0) && kernel_ready(h, v, tn, nrhs) == kSolveRows) {
         MixTable *mt = nullptr;
         for (int r0 = 0; r0 < nrhs; r0 += 32) {
             const int nb = nrhs - r0 < 32 ? nrhs - r0 : 32;
@@ -1855,7 +1821,8 @@ extern "C" capsp_status_t capsp_solve_host(capsp_handle_t h, const void *b_host,
     const int v = view_of(h, kOpSolve);
     const long long nseg_want = ((long long)h->n + kSegmentRowsMin - 1) / kSegmentRowsMin;
     const Tuning tn = current_tuning(h, kOpSolve, nrhs);
-    const bool progressive = !chain_selected(h, v, tn) && !column_driven(h, kOpSolve) && view_level(h, v) && nseg_want >= 2 &&
+    const bool chain = kernel_wanted(h, v, tn, nrhs) == kSolveChain;
+    const bool progressive = !chain && !column_driven(h, kOpSolve) && view_level(h, v) && nseg_want >= 2 &&
                              row_hostio_supported(tn.kind < 0 ? kRowWrtFst : tn.kind, tn.R, nrhs) &&
                              wait_value32() != nullptr && pinned_alias(x_host, h->device) != nullptr;
     if (!progressive) {
@@ -1874,7 +1841,7 @@ extern "C" capsp_status_t capsp_solve_host(capsp_handle_t h, const void *b_host,
             (!column_driven(h, kOpSolve) && view_level(h, v) && !(wide_levels(h, v) && nrhs == 1))
                 ? pinned_alias(b_host, h->device)
                 : nullptr;
-        if (b_in_place && !chain_selected(h, v, tn)) {
+        if (b_in_place && !chain) {
             // the row kernels: many more rows wait for their b side by side
             h->row_kernels_only = true;
             const capsp_status_t sd = dispatch(h, kOpSolve, b_in_place, dx, nullptr, nullptr, nrhs, nrhs, st);
@@ -1999,7 +1966,7 @@ extern "C" capsp_status_t capsp_autotune(capsp_handle_t h, const void *b, void *
         const bool allow_mix = alg == CAPSP_ALG_AUTO || alg == CAPSP_ALG_MIX;
         const int bpss[3] = {1, 2, 0};
         const Tuning base = untuned(h, kOpSolve);
-        if (chain_selected(h, v, base) || stream_wanted(h, v, base, nrhs))
+        if (kernel_wanted(h, v, base, nrhs) != kSolveRows)
             cands.push_back(base);
         if (allow_thread) {
             // the default launch shape first: the search never ends worse
@@ -2210,7 +2177,7 @@ extern "C" capsp_status_t capsp_get_info(capsp_handle_t h, capsp_info_t *info)
             info->element_occupy = mit->second.eo;
             if (alg == CAPSP_ALG_AUTO)
                 alg = mit->second.wo > 0.0 ? CAPSP_ALG_MIX : CAPSP_ALG_WRTFST;
-        } else if (chain_selected(h, v, tn) || stream_selected(h, v, tn, 1)) {
+        } else if (kernel_ready(h, v, tn, 1) != kSolveRows) {
             // these kernels need no selector table on the device; report
             // the row kernels' choice for this matrix
             std::vector<int> table((size_t)h->n + 2);

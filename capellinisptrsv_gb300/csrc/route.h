@@ -1,0 +1,70 @@
+// Which kernel solves a level-ordered view when the caller leaves the choice to
+// the library: rules on sizes, row lengths, precision and right-hand sides
+// (host-only logic, tested without the CUDA runtime).
+#pragma once
+
+namespace capsp {
+
+enum SolveKernel { kSolveRows = 0, kSolveChain = 1, kSolveStream = 2 };
+
+// Rows per level up to which the chain kernel is the faster one.  Measured on
+// GB300 in FP64, chain against row kernel: 8 rows per level (1,048,576 Zipf rows)
+// 28.3 against 100.9 ms, 13 (2,003 rows) 27 against 137 us, 115 (40,000 rows of
+// 3-12 dependencies) 162 against 460 us, 146 (38,261 rows of 3-10) 146 against 336
+// us, 200 (20,000 rows of 1-5) 57 against 92 us, 377 (60,000 rows of 1-7) 171
+// against 147 us.
+constexpr long long kChainLevelRows = 256;
+
+// Rows per level from which the stream kernel is the faster one whatever the
+// number of right-hand sides (auto_kernel)
+constexpr long long kStreamAnyRows = 12288;
+// ... and the longest row it takes: a lane walks its row 8 or 12 entries at a
+// time, so longer ones are for the mixed row kernel's warps.  (Banded matrices
+// have some of 40 to 110 entries in their transposes, where few columns precede.)
+constexpr int kStreamLongest = 128;
+
+struct ViewShape {
+    long long n = 0, levels = 0, entries = 0;  // rows, levels, off-diagonal entries
+    int longest = 0;                           // off-diagonal entries of the longest row
+    bool chain = false;                        // a launch plan of the chain kernel exists
+    bool f64 = true;
+};
+
+// whether the levels are narrow enough for the chain kernel
+inline bool chain_levels(long long n, long long levels) { return n <= kChainLevelRows * levels; }
+
+// `cols`: right-hand sides, rounded up to the lanes or lane slots they take.
+//
+// The chain kernel comes first wherever it has a plan.  Of the others, the row
+// kernels follow a chain of dependencies faster, the stream kernel gets through
+// more rows.  Measured on GB300, time of the row kernel / time of the stream
+// kernel:
+//   1 RHS: FP64 0.87 at 5.9k rows per level, 1.03 at 12k, 1.25 at 14k, 1.36 at 47k;
+//          FP32 0.92, -, 1.40, 1.42
+//   2 RHS: FP64 0.91 at 5.9k, 1.47 at 14k, 1.74 at 47k; FP32 1.00, 1.51, 1.86
+//   4 and more, FP32: 1.04 to 3.0 from 700 rows per level on
+//   4 and more, FP64: by the rows' length.  5 to 8 entries on average (12 fit a
+//          lane, 8 a lane of the row kernel): 1.05 to 1.24 from 700 rows per level
+//          on.  Shorter: 1.03 at 4.6k row-columns per level, 0.96 at 11k, 1.17 at
+//          23k, 1.10 to 1.49 above.  Longer: 0.94 at 6k, 1.10 at 12k.
+inline SolveKernel auto_kernel(const ViewShape &s, int cols)
+{
+    if (s.chain)
+        return kSolveChain;
+    if (s.longest > kStreamLongest || s.levels < 1)
+        return kSolveRows;
+    const long long rows = s.n / s.levels;  // per level
+    if (rows >= kStreamAnyRows)
+        return kSolveStream;
+    if (rows < kChainLevelRows || cols == 1)
+        return kSolveRows;
+    if (cols == 2)
+        return rows >= 8192 ? kSolveStream : kSolveRows;
+    if (!s.f64)
+        return kSolveStream;
+    if (s.entries > 8 * s.n)
+        return rows * cols >= 10240 ? kSolveStream : kSolveRows;
+    return s.entries > 5 * s.n || rows * cols >= 16384 ? kSolveStream : kSolveRows;
+}
+
+}  // namespace capsp

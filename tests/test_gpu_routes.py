@@ -1,0 +1,66 @@
+"""Solves on either side of the lines between the kernels of algorithm "auto",
+against the oracle at the suite's bars (relative infinity-norm error 1e-12 in
+FP64, 1e-5 in FP32)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import capellinisptrsv_gb300 as cs
+import oracle
+from conftest import rel_inf_err
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+TOL = {np.float64: 1e-12, np.float32: 1e-5}
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).to(DEV)
+
+
+def host(t):
+    torch.cuda.synchronize()
+    return t.cpu().numpy()
+
+
+def grid(width, levels, backs):
+    """`levels` levels of `width` rows: row i depends on the rows `backs` before it, the
+    nearest of them `width` before."""
+    n = width * levels
+    rows, cols = [], []
+    for d in backs:
+        i = np.arange(d, n)
+        rows.append(i)
+        cols.append(i - d)
+    i = np.arange(n)
+    rows, cols = np.concatenate(rows + [i]), np.concatenate(cols + [i])
+    order = np.argsort(rows * (n + 1.0) + cols, kind="stable")
+    rows, cols = rows[order], cols[order]
+    v = np.random.default_rng(width).uniform(-1.0, 1.0, len(rows))
+    d = rows == cols
+    v[d] = 0.0
+    v[d] = 1.0 + np.bincount(rows, np.abs(v), minlength=n)
+    rp = np.zeros(n + 1, np.int32)
+    rp[1:] = np.cumsum(np.bincount(rows, minlength=n))
+    return cs.CSRMatrix(n, rp, cols.astype(np.int32), v)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("width", [255, 256, 257])
+def test_either_side_of_the_chain_kernels_line(width, dtype):
+    """Rows of 2 and of 6 dependencies, some beyond the ring; more right-hand sides after fewer."""
+    for backs in ((width, 12 * width), tuple(width * t + 3 * (t > 1) * t for t in (1, 2, 3, 5, 9, 14))):
+        m = grid(width, 100, backs)
+        v = m.val.astype(dtype)
+        s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(v))
+        assert s.info()["levels"] == 100
+        for k in (1, 3, 16, 33):
+            b = np.random.default_rng(k).standard_normal((m.n, k)).astype(dtype)
+            xo = oracle.solve_csr_lower(m.rowptr, m.colidx, v, b)
+            yo = oracle.solve_csr_transpose(m.rowptr, m.colidx, v, b)
+            assert rel_inf_err(host(s.solve(dev(b))), xo) <= TOL[dtype], k
+            assert rel_inf_err(host(s.solve_transpose(dev(b))), yo) <= TOL[dtype], k
+        s.status()

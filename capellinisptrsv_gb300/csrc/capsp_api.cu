@@ -93,7 +93,7 @@ struct ChainPlan {
 // Layout of the stream kernel over a view (kernels_stream.cuh); built at analysis
 // where every solve takes it, else before the first solve that does
 struct StreamPlan {
-    bool tried = false;  // built, or found unsuitable
+    bool tried = false;  // built, found unsuitable, or barred by a captured refresh
     bool ok = false;
     int nslices = 0;
     void *d_all = nullptr;  // the arrays below
@@ -355,6 +355,15 @@ static capsp_status_t launch_view_refresh(capsp_handle_t h, const RowView &rv, i
     else
         CAPSP_CUDA(launch_level_values<float>(rv.d_lptr, rv.d_lsrc, rv.d_dsrc, h->n, (const float *)h->d_val,
                                               (float *)rv.d_lval, (float *)rv.d_linv, bad, st));
+    return CAPSP_OK;
+}
+
+// whether work enqueued on `st` goes into a caller's capture
+static capsp_status_t is_capturing(cudaStream_t st, bool *yes)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CAPSP_CUDA(cudaStreamIsCapturing(st, &cs));
+    *yes = cs != cudaStreamCaptureStatusNone;
     return CAPSP_OK;
 }
 
@@ -632,7 +641,6 @@ static capsp_status_t build_view(capsp_handle_t h, int v)
         CAPSP_CUDA(cudaMalloc(&rv.d_lnear, sizeof(int) * (size_t)n));
         CAPSP_CUDA(cudaMemcpy(rv.d_lnear, lnear.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice));
     }
-    free_stream(rv.stream);
     rv.h_levels.assign(level_start.begin() + 1, level_start.begin() + levels + 2);
     // levels narrower than ~4k rows: two resident warps per SM for the row
     // path by default (more rows in flight than a few levels only add pollers)
@@ -861,6 +869,13 @@ extern "C" capsp_status_t capsp_refresh_values(capsp_handle_t h, const void *val
     }
     const int dl = diag_last_of(h->format, h->uplo);
     cudaStream_t st = (cudaStream_t)stream;
+    bool captured = false;
+    CAPSP_TRY(is_capturing(st, &captured));
+    // a captured refresh gives new values, whenever it is replayed, to what exists
+    // now: a stream layout built later would keep its old ones, so none is
+    if (captured)
+        for (RowView &rv : h->view)
+            rv.stream.tried = true;
     int *bad = h->d_err + 3;  // sticky diagnostic slot: first row with a bad diagonal
     if (h->dtype == CAPSP_R_64F)
         CAPSP_CUDA(launch_inv_diag<double>(h->d_ptr, (const double *)h->d_val, (double *)h->d_inv, h->n, dl, bad, st));
@@ -1397,13 +1412,13 @@ static capsp_status_t enqueue_rows(capsp_handle_t h, int v, const T *b, T *x, in
         if (kernel == kSolveStream) {
             // a caller's capture that started before the layout was built goes
             // on with the row kernels
-            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            bool captured = false;
             const int cols = lanes_for_rhs(nrhs < 32 ? nrhs : 32);
             if (!rv.stream.tried || (rv.stream.ok && rv.stream.pub_cap < cols))
-                CAPSP_CUDA(cudaStreamIsCapturing(st, &cs));
-            if (cs == cudaStreamCaptureStatusNone)
+                CAPSP_TRY(is_capturing(st, &captured));
+            if (!captured)
                 CAPSP_TRY(ensure_stream(h, v, nrhs));
-            if (cs != cudaStreamCaptureStatusNone || !rv.stream.ok)
+            if (captured || !rv.stream.ok)
                 kernel = kSolveRows;
         }
         if (kernel != kSolveStream)

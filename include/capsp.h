@@ -171,7 +171,10 @@ capsp_status_t capsp_set_values(capsp_handle_t h, const void *val);
  * with val = NULL, keep the current pointer) and recompute 1/diag on `stream`
  * without synchronising.  Meant for values that change between solves, e.g.
  * parameters updated in place by an optimiser; a zero diagonal then shows up
- * as inf/NaN in the results instead of an error code. */
+ * as inf/NaN in the results instead of an error code.  It may be captured: a
+ * replay then refreshes what the handle held at capture time, so capsp_reserve
+ * belongs before the capture (a stream layout that does not exist by then is
+ * not built any more, and the row kernels solve in its place). */
 capsp_status_t capsp_refresh_values(capsp_handle_t h, const void *val, void *stream);
 
 capsp_status_t capsp_destroy(capsp_handle_t h);

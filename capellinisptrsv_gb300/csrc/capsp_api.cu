@@ -120,6 +120,7 @@ struct RowView {
     int *d_lnear = nullptr;   // first near entry per position (chain.ok only)
     ChainPlan chain;
     StreamPlan stream;
+    bool late = false;  // built after a refresh was captured: its values are refreshed before every solve
     std::vector<int> h_levels;  // first position of every level, and n
     std::vector<int> h_lcum;  // lptr[k] + k: row-count prefix in position space (mix tables)
     // capsp_solve_host's b upload: highest b segment per 32 positions (kernel: b_group_seg)
@@ -207,6 +208,7 @@ struct capsp_handle_s {
     size_t l2_prev_limit = 0;  // persisting carve-out before this handle changed it
     size_t l2_window = 0;      // largest window the device accepts
     size_t l2_persist = 0;     // persisting carve-out this handle asked for
+    bool refresh_captured = false;  // a caller's capture holds a value refresh
     bool row_kernels_only = false;  // capsp_hop_latency; capsp_solve_host while b or x is on its way
     int sched = CAPSP_SCHED_LEVEL;  // schedule of view 0; view 1 is always level-ordered
     RowView view[2];
@@ -646,6 +648,7 @@ static capsp_status_t build_view(capsp_handle_t h, int v)
     // path by default (more rows in flight than a few levels only add pollers)
     rv.narrow = (long long)n < 4096LL * (long long)levels;
     rv.built = true;
+    rv.late = h->refresh_captured;
     int *d_bad = nullptr;
     CAPSP_CUDA(cudaMalloc(&d_bad, sizeof(int)));
     const int big = INT_MAX;
@@ -873,9 +876,11 @@ extern "C" capsp_status_t capsp_refresh_values(capsp_handle_t h, const void *val
     CAPSP_TRY(is_capturing(st, &captured));
     // a captured refresh gives new values, whenever it is replayed, to what exists
     // now: a stream layout built later would keep its old ones, so none is
-    if (captured)
+    if (captured) {
+        h->refresh_captured = true;
         for (RowView &rv : h->view)
             rv.stream.tried = true;
+    }
     int *bad = h->d_err + 3;  // sticky diagnostic slot: first row with a bad diagonal
     if (h->dtype == CAPSP_R_64F)
         CAPSP_CUDA(launch_inv_diag<double>(h->d_ptr, (const double *)h->d_val, (double *)h->d_inv, h->n, dl, bad, st));
@@ -1423,6 +1428,8 @@ static capsp_status_t enqueue_rows(capsp_handle_t h, int v, const T *b, T *x, in
         }
         if (kernel != kSolveStream)
             CAPSP_TRY(ensure_xp(h, nrhs));
+        if (rv.late)
+            CAPSP_TRY(launch_view_refresh(h, rv, h->d_err + 3, st));
     }
     for (int r0 = 0; r0 < nrhs; r0 += 32) {
         const int nb = nrhs - r0 < 32 ? nrhs - r0 : 32;

@@ -50,3 +50,29 @@ def test_captured_refresh_reaches_every_later_solve():
         assert rel_inf_err(host(x1), oracle.solve_csr_lower(m.rowptr, m.colidx, v, b1)) <= 1e-12
         assert rel_inf_err(host(s.solve(bd16)), oracle.solve_csr_lower(m.rowptr, m.colidx, v, b16)) <= 1e-12
     s.status()
+
+
+@pytest.mark.parametrize("k", [1, 16])
+def test_transpose_built_after_a_captured_refresh_follows_it(k):
+    """The transposed view does not exist when the refresh is captured."""
+    m = blocks(30, 701, 3, 10, 8)
+    val = dev(m.val)
+    b = np.random.default_rng(k).standard_normal((m.n, k))
+    bd = dev(b)
+    x = torch.empty_like(bd)
+    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), val)
+    s.solve(bd, x)
+
+    def step():
+        s.refresh_values(val)
+        s.solve(bd, x)
+
+    g = capture(step)
+    assert rel_inf_err(host(s.solve_transpose(bd)),
+                       oracle.solve_csr_transpose(m.rowptr, m.colidx, m.val, b)) <= 1e-12
+    v = m.val * np.where(np.arange(m.nnz) % 2 == 0, 1.5, 2.0)
+    val.copy_(dev(v))
+    g.replay()
+    assert rel_inf_err(host(x), oracle.solve_csr_lower(m.rowptr, m.colidx, v, b)) <= 1e-12
+    assert rel_inf_err(host(s.solve_transpose(bd)), oracle.solve_csr_transpose(m.rowptr, m.colidx, v, b)) <= 1e-12
+    s.status()

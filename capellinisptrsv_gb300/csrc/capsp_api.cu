@@ -208,6 +208,14 @@ struct capsp_handle_s {
     size_t l2_prev_limit = 0;  // persisting carve-out before this handle changed it
     size_t l2_window = 0;      // largest window the device accepts
     size_t l2_persist = 0;     // persisting carve-out this handle asked for
+    // A caller's capture holds solves of this handle, whose graphs point at the
+    // scratch of that time: what a larger one replaces is kept until the end
+    // (kMaxRetired: from then on scratch grows by powers of two up to 32).
+    static constexpr int kMaxRetired = 24;
+    bool solve_captured = false;
+    bool own_capture = false;  // capsp_graph_solve's: its graphs are dropped when scratch changes
+    void *retired[kMaxRetired] = {};
+    int num_retired = 0;
     bool refresh_captured = false;  // a caller's capture holds a value refresh
     bool row_kernels_only = false;  // capsp_hop_latency; capsp_solve_host while b or x is on its way
     int sched = CAPSP_SCHED_LEVEL;  // schedule of view 0; view 1 is always level-ordered
@@ -265,6 +273,8 @@ static void free_handle(capsp_handle_t h)
         free_stream(rv.stream);
     }
     cudaFree(h->d_xp);
+    for (int k = 0; k < h->num_retired; ++k)
+        cudaFree(h->retired[k]);
     if (h->stage_stream)
         cudaStreamDestroy(h->stage_stream);
     if (h->copy_stream)
@@ -360,11 +370,12 @@ static capsp_status_t launch_view_refresh(capsp_handle_t h, const RowView &rv, i
     return CAPSP_OK;
 }
 
-// whether work enqueued on `st` goes into a caller's capture
+// whether work enqueued on `st` goes into a capture
 static capsp_status_t is_capturing(cudaStream_t st, bool *yes)
 {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    CAPSP_CUDA(cudaStreamIsCapturing(st, &cs));
+    if (st != 0)  // the default stream cannot be captured
+        CAPSP_CUDA(cudaStreamIsCapturing(st, &cs));
     *yes = cs != cudaStreamCaptureStatusNone;
     return CAPSP_OK;
 }
@@ -1224,10 +1235,21 @@ static Tuning current_tuning(capsp_handle_t h, Op op, int nrhs)
 // enqueue paths
 // ---------------------------------------------------------------------------
 
+// give up scratch that a larger one replaces
+static void retire(capsp_handle_t h, void *p)
+{
+    if (p == nullptr)
+        return;
+    if (h->solve_captured && h->num_retired < capsp_handle_s::kMaxRetired)
+        h->retired[h->num_retired++] = p;
+    else
+        cudaFree(p);
+}
+
 // position-ordered publication scratch for the level schedule
 static capsp_status_t ensure_xp(capsp_handle_t h, int nrhs)
 {
-    const int want = nrhs < 32 ? nrhs : 32;
+    int want = nrhs < 32 ? nrhs : 32;
     if (h->xp_cap < want) {
         h->graphs.invalidate();  // captured row solves point at the old scratch
         // After warm-up solves of as many right-hand sides in the stream kernel, which
@@ -1236,11 +1258,12 @@ static capsp_status_t ensure_xp(capsp_handle_t h, int nrhs)
         bool warm = false;
         for (const RowView &rv : h->view)
             warm = warm || rv.stream.pub_cap >= want;
+        if (h->solve_captured)
+            want = lanes_for_rhs(want);
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         if (warm)
             CAPSP_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-        if (h->d_xp)
-            cudaFree(h->d_xp);
+        retire(h, h->d_xp);
         h->d_xp = nullptr;
         h->xp_cap = 0;
         const cudaError_t e = cudaMalloc(&h->d_xp, h->vbytes * (size_t)h->n * (size_t)want);
@@ -1261,20 +1284,36 @@ static capsp_status_t ensure_stream(capsp_handle_t h, int v, int nrhs)
     const int want = lanes_for_rhs(nrhs < 32 ? nrhs : 32);
     if (sp.ok && sp.pub_cap < want) {
         h->graphs.invalidate();  // captured stream solves point at the old scratch
-        cudaFree(sp.d_pub);
-        sp.d_pub = nullptr;
-        sp.pub_cap = 0;
-        const cudaError_t e = cudaMalloc(&sp.d_pub, h->vbytes * 8 * (size_t)sp.nslices * (size_t)want);
-        if (e == cudaErrorMemoryAllocation) {  // no room: the row kernels' scratch is smaller
+        if (!h->solve_captured) {
+            cudaFree(sp.d_pub);
+            sp.d_pub = nullptr;
+            sp.pub_cap = 0;
+        }
+        void *d = nullptr;
+        const cudaError_t e = cudaMalloc(&d, h->vbytes * 8 * (size_t)sp.nslices * (size_t)want);
+        if (e == cudaErrorMemoryAllocation) {
+            // no room: the row kernels' scratch is smaller.  The layout goes too,
+            // unless a captured solve or refresh points at it.
             cudaGetLastError();
-            free_stream(sp);
-            sp.tried = true;
+            if (!h->solve_captured && !h->refresh_captured) {
+                free_stream(sp);
+                sp.tried = true;
+            }
             return CAPSP_OK;
         }
         CAPSP_CUDA(e);
+        retire(h, sp.d_pub);
+        sp.d_pub = d;
         sp.pub_cap = want;
     }
     return CAPSP_OK;
+}
+
+// whether a solve of nrhs right-hand sides can go through the stream layout of view v
+static bool stream_ready(capsp_handle_t h, int v, int nrhs)
+{
+    const StreamPlan &sp = h->view[v].stream;
+    return sp.ok && sp.pub_cap >= lanes_for_rhs(nrhs < 32 ? nrhs : 32);
 }
 
 // The kernel that a row-driven solve over view v, whose level layout is built, asks
@@ -1296,13 +1335,6 @@ static SolveKernel kernel_wanted(capsp_handle_t h, int v, const Tuning &tn, int 
     s.f64 = h->dtype == CAPSP_R_64F;
     const SolveKernel k = auto_kernel(s, lanes_for_rhs(nrhs < 32 ? nrhs : 32));
     return k == kSolveStream && h->stuck_row >= 0 ? kSolveRows : k;
-}
-
-// ... and the one it runs in, as far as the stream layout has been built
-static SolveKernel kernel_ready(capsp_handle_t h, int v, const Tuning &tn, int nrhs)
-{
-    const SolveKernel k = kernel_wanted(h, v, tn, nrhs);
-    return k == kSolveStream && !h->view[v].stream.ok ? kSolveRows : k;
 }
 
 // stream kernel over view v, right-hand sides [0, nb) of b and x
@@ -1411,19 +1443,19 @@ static capsp_status_t enqueue_rows(capsp_handle_t h, int v, const T *b, T *x, in
     RowView &rv = h->view[v];
     // decided once: the scratch below is that of the kernel that runs
     SolveKernel kernel = kSolveRows;
+    bool captured = false;
     if (level) {
+        CAPSP_TRY(is_capturing(st, &captured));
+        if (captured && !h->own_capture)
+            h->solve_captured = true;
         CAPSP_TRY(build_view(h, v));
         kernel = kernel_wanted(h, v, tn, nrhs);
         if (kernel == kSolveStream) {
             // a caller's capture that started before the layout was built goes
             // on with the row kernels
-            bool captured = false;
-            const int cols = lanes_for_rhs(nrhs < 32 ? nrhs : 32);
-            if (!rv.stream.tried || (rv.stream.ok && rv.stream.pub_cap < cols))
-                CAPSP_TRY(is_capturing(st, &captured));
-            if (!captured)
+            if (!captured && !stream_ready(h, v, nrhs))
                 CAPSP_TRY(ensure_stream(h, v, nrhs));
-            if (captured || !rv.stream.ok)
+            if (!stream_ready(h, v, nrhs))
                 kernel = kSolveRows;
         }
         if (kernel != kSolveStream)
@@ -1699,12 +1731,17 @@ static capsp_status_t prepare(capsp_handle_t h, int nrhs, Op op)
     if (view_level(h, v))
         CAPSP_TRY(build_view(h, v));
     const Tuning tn = current_tuning(h, op, nrhs);
+    SolveKernel kernel = kSolveRows;
     if (view_level(h, v)) {
-        if (kernel_wanted(h, v, tn, nrhs) == kSolveStream)
+        kernel = kernel_wanted(h, v, tn, nrhs);
+        if (kernel == kSolveStream) {
             CAPSP_TRY(ensure_stream(h, v, nrhs));
+            if (!stream_ready(h, v, nrhs))
+                kernel = kSolveRows;
+        }
         CAPSP_TRY(ensure_xp(h, nrhs));  // fewer right-hand sides may go to the row kernels
     }
-    if ((tn.kind == kRowMix || tn.kind < 0) && kernel_ready(h, v, tn, nrhs) == kSolveRows) {
+    if ((tn.kind == kRowMix || tn.kind < 0) && kernel == kSolveRows) {
         MixTable *mt = nullptr;
         for (int r0 = 0; r0 < nrhs; r0 += 32) {
             const int nb = nrhs - r0 < 32 ? nrhs - r0 : 32;
@@ -2094,7 +2131,9 @@ extern "C" capsp_status_t capsp_graph_solve(capsp_handle_t h, const void *b, voi
     cudaGraphExec_t *exec_p = h->graphs.find(key);
     if (!exec_p) {
         CAPSP_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        h->own_capture = true;
         capsp_status_t s = dispatch(h, kOpSolve, b, x, nullptr, nullptr, nrhs, ld, st);
+        h->own_capture = false;
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(st, &graph);
         if (s != CAPSP_OK) {
@@ -2199,7 +2238,8 @@ extern "C" capsp_status_t capsp_get_info(capsp_handle_t h, capsp_info_t *info)
             info->element_occupy = mit->second.eo;
             if (alg == CAPSP_ALG_AUTO)
                 alg = mit->second.wo > 0.0 ? CAPSP_ALG_MIX : CAPSP_ALG_WRTFST;
-        } else if (kernel_ready(h, v, tn, 1) != kSolveRows) {
+        } else if (kernel_wanted(h, v, tn, 1) == kSolveChain ||
+                   (kernel_wanted(h, v, tn, 1) == kSolveStream && h->view[v].stream.ok)) {
             // these kernels need no selector table on the device; report
             // the row kernels' choice for this matrix
             std::vector<int> table((size_t)h->n + 2);

@@ -76,3 +76,31 @@ def test_transpose_built_after_a_captured_refresh_follows_it(k):
     assert rel_inf_err(host(x), oracle.solve_csr_lower(m.rowptr, m.colidx, v, b)) <= 1e-12
     assert rel_inf_err(host(s.solve_transpose(bd)), oracle.solve_csr_transpose(m.rowptr, m.colidx, v, b)) <= 1e-12
     s.status()
+
+
+@pytest.mark.parametrize("eager", [(), (2, 5, 32)])
+def test_captured_solves_keep_their_scratch(eager):
+    """One right-hand side takes the row kernels, 16 the stream kernel, 8 the row kernels
+    again, with larger scratch: first needed inside a capture whose graph, like an
+    earlier one, points at the smaller.  `eager`: row-kernel solves that outgrow it later."""
+    m = blocks(12, 1_500, 1, 6, 9)
+    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(m.val))
+    rng = np.random.default_rng(9)
+    b = {k: rng.standard_normal((m.n, k)) for k in (1, 8, 16)}
+    bd = {k: dev(b[k]) for k in b}
+    x = {k: torch.empty_like(bd[k]) for k in b}
+    want = {k: oracle.solve_csr_lower(m.rowptr, m.colidx, m.val, b[k]) for k in b}
+    for k in (1, 16):
+        s.solve(bd[k], x[k])
+    first = capture(lambda: s.solve(bd[1], x[1]))
+    second = capture(lambda: (s.solve(bd[1], x[1]), s.solve(bd[8], x[8])))
+    s.set_algorithm("wrtfst")
+    for k in eager:
+        s.solve(dev(rng.standard_normal((m.n, k))))
+    for g, ks in ((first, (1,)), (second, (1, 8)), (first, (1,))):
+        for k in ks:
+            x[k].zero_()
+        g.replay()
+        for k in ks:
+            assert rel_inf_err(host(x[k]), want[k]) <= 1e-12
+    s.status()

@@ -641,7 +641,8 @@ cudaError_t launch_chain_solve(const ChainArgs<T> &a, int nrhs, cudaStream_t st)
     const size_t staged = (size_t)kChainWarps * chain_slot_bytes<T>(a.entries);
     const size_t chain = (size_t)a.ring * sizeof(T) + 16 + (size_t)a.slots * chain_slot_bytes<T>(a.entries);
     const size_t smem = kChainRing + (staged > chain ? staged : chain) + 16;  // the last slot's look-ahead
-    cudaError_t e = cudaFuncSetAttribute(chain_solve_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit is the kernel's, not the launch's: one value for all handles and threads
+    cudaError_t e = cudaFuncSetAttribute(chain_solve_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kChainSmem);
     if (e != cudaSuccess)
         return e;
     cudaLaunchAttribute at = {};

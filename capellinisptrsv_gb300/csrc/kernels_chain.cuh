@@ -377,6 +377,7 @@ __device__ __forceinline__ void chain_feed(const ChainArgs<T> &a, unsigned base,
         }
         if (__any_sync(kFullMask, late))
             return;
+        __syncwarp();  // the sums above are other lanes' (a vote orders no memory)
         const unsigned nv = ((unsigned)total * (unsigned)sizeof(T) + 15u) / 16u;
         const unsigned ni = ((unsigned)total * 2u + 15u) / 16u;
         const unsigned vo = hdr / 16u, io = vo + (unsigned)a.entries * (unsigned)sizeof(T) / 16u;
@@ -419,6 +420,7 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
                 if (__any_sync(kFullMask, rw.expired(a.wait, a.err, p)))
                     return;
             __threadfence_block();
+            __syncwarp();  // every lane overwrites what the warps that were seen to be done have read
             ring_store(ring_at + (unsigned)sizeof(U) * (((unsigned)p + 32u * (unsigned)a.ahead) & mask), VB::kPending);
         }
         {

@@ -228,8 +228,8 @@ __device__ __forceinline__ float chain_fold(float v, float u, float acc, float &
 __device__ __forceinline__ double chain_sum(double acc, double) { return acc; }
 __device__ __forceinline__ float chain_sum(float acc, float low)
 {
-    const float sum = acc + low;
-    return sum == sum ? sum : acc;  // an infinite sum has no remainder (infinity - infinity)
+    // where a sum or a step of its remainder overflowed there is none to add
+    return fabsf(low) <= 3.402823466e38f ? acc + low : acc;
 }
 
 // Feeder: chunks c = s, s + step, ... of one slot.

@@ -64,3 +64,21 @@ def test_either_side_of_the_chain_kernels_line(width, dtype):
             assert rel_inf_err(host(s.solve(dev(b))), xo) <= TOL[dtype], k
             assert rel_inf_err(host(s.solve_transpose(dev(b))), yo) <= TOL[dtype], k
         s.status()
+
+
+def test_fp32_products_beyond_the_range_that_cancel():
+    """b/d of -3e38 and a product of 4e38: the fused sum is 1e38, and so is the solve's
+    (its remainder has no finite value).  Two levels of 64 rows: the chain kernel."""
+    n = 128
+    i = np.arange(n)
+    rp = np.concatenate([i[:65], 64 + 2 * (i[:64] + 1)]).astype(np.int32)
+    ci = np.concatenate([i[:64], np.stack([i[:64], i[64:]], 1).ravel()]).astype(np.int32)
+    v = np.concatenate([np.ones(64), np.tile([-2.0, 1.0], 64)]).astype(np.float32)
+    b = np.concatenate([np.full(64, 2e38), np.full(64, -3e38)]).astype(np.float32)
+    s = cs.TriangularSolver(dev(rp), dev(ci), dev(v))
+    x = host(s.solve(dev(b)))
+    xo = oracle.solve_csr_lower(rp, ci, v.astype(np.float64), b.astype(np.float64))
+    assert rel_inf_err(x, xo) <= 1e-5
+    s.set_algorithm("wrtfst")
+    assert rel_inf_err(host(s.solve(dev(b))), xo) <= 1e-5
+    s.status()

@@ -1317,9 +1317,8 @@ static bool stream_ready(capsp_handle_t h, int v, int nrhs)
 }
 
 // The kernel that a row-driven solve over view v, whose level layout is built, asks
-// for (auto_kernel): AUTO with the default launch shape, outside the debug and
-// L2-window modes; the debug hook of a row that never publishes keeps a solve that
-// the stream kernel would take on the row kernels.
+// for (auto_kernel): AUTO with the default launch shape, outside the tracing and
+// L2-window modes.
 static SolveKernel kernel_wanted(capsp_handle_t h, int v, const Tuning &tn, int nrhs)
 {
     const RowView &rv = h->view[v];
@@ -1333,8 +1332,19 @@ static SolveKernel kernel_wanted(capsp_handle_t h, int v, const Tuning &tn, int 
     s.longest = rv.longest;
     s.chain = rv.chain.ok;
     s.f64 = h->dtype == CAPSP_R_64F;
-    const SolveKernel k = auto_kernel(s, lanes_for_rhs(nrhs < 32 ? nrhs : 32));
-    return k == kSolveStream && h->stuck_row >= 0 ? kSolveRows : k;
+    return auto_kernel(s, lanes_for_rhs(nrhs < 32 ? nrhs : 32));
+}
+
+// Where row `row` is in a stream layout (debug hook of a row that never publishes;
+// the kernel has no test for it, which cost 1 % on narrow levels).  Synchronous.
+static capsp_status_t find_in_stream(int row, const StreamPlan &sp, int *pos)
+{
+    const size_t np = 8 * (size_t)sp.nslices;
+    std::vector<int> rows(np);
+    CAPSP_CUDA(cudaDeviceSynchronize());  // an earlier solve may have it hidden
+    CAPSP_CUDA(cudaMemcpy(rows.data(), sp.d_row, sizeof(int) * np, cudaMemcpyDeviceToHost));
+    *pos = (int)(std::find(rows.begin(), rows.end(), row) - rows.begin());
+    return *pos < (int)np ? CAPSP_OK : fail(CAPSP_ERR_INVALID, "row %d is not in the layout", row);
 }
 
 // stream kernel over view v, right-hand sides [0, nb) of b and x
@@ -1361,6 +1371,12 @@ static capsp_status_t enqueue_stream(capsp_handle_t h, int v, const T *b, T *x, 
     a.words = h->d_ticket;
     a.err = h->d_err;
     a.wait = h->wait;
+    int stuck_pos = -1;
+    if (h->stuck_row >= 0) {
+        CAPSP_TRY(find_in_stream(h->stuck_row, sp, &stuck_pos));
+        const int hidden = stream_unpublished(h->stuck_row);  // for this solve
+        CAPSP_CUDA(cudaMemcpyAsync(sp.d_row + stuck_pos, &hidden, sizeof(int), cudaMemcpyHostToDevice, st));
+    }
     const bool prof = h->profiling && first;
     if (prof)
         CAPSP_CUDA(cudaEventRecord(h->ev_k0, st));
@@ -1380,6 +1396,8 @@ static capsp_status_t enqueue_stream(capsp_handle_t h, int v, const T *b, T *x, 
     CAPSP_CUDA(launch_stream_solve<T>(a, long_rows, pairs, warps, h->num_sms, st));
     if (prof)
         CAPSP_CUDA(cudaEventRecord(h->ev_k1, st));
+    if (stuck_pos >= 0)
+        CAPSP_CUDA(cudaMemcpyAsync(sp.d_row + stuck_pos, &h->stuck_row, sizeof(int), cudaMemcpyHostToDevice, st));
     return CAPSP_OK;
 }
 
@@ -1455,7 +1473,7 @@ static capsp_status_t enqueue_rows(capsp_handle_t h, int v, const T *b, T *x, in
             // on with the row kernels
             if (!captured && !stream_ready(h, v, nrhs))
                 CAPSP_TRY(ensure_stream(h, v, nrhs));
-            if (!stream_ready(h, v, nrhs))
+            if (!stream_ready(h, v, nrhs) || (captured && h->stuck_row >= 0))
                 kernel = kSolveRows;
         }
         if (kernel != kSolveStream)

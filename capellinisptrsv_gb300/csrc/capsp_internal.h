@@ -103,12 +103,18 @@ struct ChainArgs {
     int stuck_row;
 };
 
+// A row that the stream kernel passes over (debug hook), as its layout names it; and back
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int stream_unpublished(int row) { return -2 - row; }
+
 // Arguments of the stream kernel (kernels_stream.cuh)
 template <typename T>
 struct StreamArgs {
     const int2 *slice;  // first entry, entries of the longest row
     long long npos;     // positions, 8 per slice
-    const int *row;     // row of every position (-1: none)
+    const int *row;     // row of every position (-1: none, below: stream_unpublished)
     const T *linv;      // 1 / diagonal of every position
     const int *idx;     // entry's position (-1: padding)
     const T *val;       // entry's value, pre-scaled to -v / diagonal

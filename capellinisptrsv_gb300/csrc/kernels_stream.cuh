@@ -78,12 +78,43 @@ __device__ __forceinline__ void stream_publish(unsigned *p, const unsigned (&v)[
                  : "memory");
 }
 
+// Spin (capsp_device.cuh) whose clock starts anew where `it` was set back to 0: the
+// budget is a single wait's, and lanes that are done never look at the clock
+struct StreamSpin {
+    unsigned it;
+    unsigned long long t0;
+    __device__ __forceinline__ StreamSpin() : it(0), t0(0) {}
+    __device__ __forceinline__ bool next(int *err, const WaitCfg &w, int row)
+    {
+        ++it;
+        if (it > 4u && w.sleep_max_ns) {
+            unsigned s = 32u << (it - 5u < 6u ? it - 5u : 6u);
+            __nanosleep(s < w.sleep_max_ns ? s : w.sleep_max_ns);
+        }
+        if ((it & 15u) == 0u) {
+            if (ld_relaxed(reinterpret_cast<const unsigned *>(err)) != 0u)
+                return true;
+            const unsigned long long now = global_timer_ns();
+            if (it == 16u) {
+                t0 = now;
+            } else if (now - t0 > w.timeout_ns || it > w.max_iters) {
+                if (atomicCAS(err + kErrStatus, 0, kStatusTimeout) == 0) {
+                    err[kErrRow] = row;
+                    err[kErrWaitedOn] = -1;
+                }
+                return true;
+            }
+        }
+        return false;
+    }
+};
+
 // A lane's row, as far as it is loaded ahead of time
 template <typename T, int TB>
 struct StreamRow {
     int at;   // first entry
     int len;  // entries, with its slice's padding
-    int row;  // -1: none
+    int row;  // < 0: none
     T dinv;
     int idx[TB];
 };
@@ -221,7 +252,7 @@ __device__ __forceinline__ void stream_rows(const StreamArgs<T> &a)
         };
         take_stock();
         bool open = mine;
-        Spin sp;
+        StreamSpin sp;
         for (;;) {
             // single precision folds a row when all of it has arrived; an FP64 FMA
             // takes so long that the part that has arrived is folded meanwhile
@@ -273,8 +304,16 @@ __device__ __forceinline__ void stream_rows(const StreamArgs<T> &a)
             }
             if (!__any_sync(kFullMask, open))
                 break;
-            if (sp.next(a.err, a.wait, cur.row, -1) && open) {
+            if (sp.next(a.err, a.wait, cur.row) && open) {
                 // give up: a quiet NaN, so that the dependants end too
+                if (a.err[kErrRow] == cur.row && a.err[kErrWaitedOn] < 0) {
+                    int q = -1;
+#pragma unroll
+                    for (int t = TB - 1; t >= 0; --t)
+                        q = (pend >> t) & 1u ? cur.idx[t] : q;
+                    const int on = q >= 0 ? a.row[q] : -1;
+                    a.err[kErrWaitedOn] = on < -1 ? stream_unpublished(on) : on;
+                }
                 U out[R];
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
@@ -301,6 +340,9 @@ __device__ __forceinline__ void stream_rows(const StreamArgs<T> &a)
                 got |= ((ask >> t) & 1u) && !late ? 1u << t : 0u;
             }
             pend &= ~got;
+            // the budget is a single wait's, and a lane that is done has none (its
+            // count stays below the first look at the clock)
+            sp.it = got || !open ? 0u : sp.it;
         }
         p = p1;
         p1 = p2;

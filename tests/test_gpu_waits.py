@@ -1,0 +1,45 @@
+"""Dependency waits that run out of their budget: what is reported, in every kernel."""
+from __future__ import annotations
+
+import re
+
+import numpy as np
+import pytest
+
+import capellinisptrsv_gb300 as cs
+import oracle
+from conftest import rel_inf_err
+from test_gpu_stream import blocks, dev, host
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def reported(m, s, b, stuck):
+    """(row, row it waited on) of a solve in which row `stuck` never publishes; the next solve is clean."""
+    xo = oracle.solve_csr_lower(m.rowptr, m.colidx, m.val, b)
+    s.debug_stuck_row(stuck, timeout_s=0.02)
+    s.solve(dev(b))
+    with pytest.raises(cs.CapspError) as e:
+        s.status()
+    assert e.value.status == 2
+    s.debug_stuck_row(-1, timeout_s=10.0)
+    assert rel_inf_err(host(s.solve(dev(b))), xo) <= 1e-12
+    s.status()
+    return tuple(int(v) for v in re.search(r"row/column (-?\d+) waiting on (-?\d+)", str(e.value)).groups())
+
+
+def check(m, got, stuck):
+    row, on = got
+    deps = m.colidx[m.rowptr[row]:m.rowptr[row + 1] - 1]
+    assert 0 <= row < m.n and (on in deps or row == on == stuck), (row, on, deps)
+
+
+@pytest.mark.parametrize("k", [1, 4, 16])
+def test_stream_reports_the_waiting_row(k):
+    """Not a lane of the same warp that is done, and not padding."""
+    m = blocks(6, 12_301, 3, 11, 12)
+    stuck = int(m.colidx[m.rowptr[15_000]])
+    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(m.val))
+    b = np.random.default_rng(k).standard_normal((m.n, k))
+    check(m, reported(m, s, b, stuck), stuck)

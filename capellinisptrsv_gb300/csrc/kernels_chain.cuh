@@ -229,7 +229,8 @@ __device__ __forceinline__ double chain_sum(double acc, double) { return acc; }
 __device__ __forceinline__ float chain_sum(float acc, float low)
 {
     // where a sum or a step of its remainder overflowed there is none to add
-    return fabsf(low) <= 3.402823466e38f ? acc + low : acc;
+    const float sum = acc + low;
+    return fabsf(sum) <= 3.402823466e38f ? sum : acc;
 }
 
 // Feeder: chunks c = s, s + step, ... of one slot.

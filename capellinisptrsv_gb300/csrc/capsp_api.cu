@@ -213,6 +213,8 @@ struct capsp_handle_s {
     // (kMaxRetired: from then on scratch grows by powers of two up to 32).
     static constexpr int kMaxRetired = 24;
     bool solve_captured = false;
+    int wait_view = -1;  // view of the latest level-ordered solve (-1: another kind), whose waits ...
+    int wait_ring = 0;   // ... name positions (row kernels: 0) or chain_code()s (chain kernel: its ring)
     bool own_capture = false;  // capsp_graph_solve's: its graphs are dropped when scratch changes
     void *retired[kMaxRetired] = {};
     int num_retired = 0;
@@ -1459,6 +1461,7 @@ static capsp_status_t enqueue_rows(capsp_handle_t h, int v, const T *b, T *x, in
 {
     const bool level = view_level(h, v);
     RowView &rv = h->view[v];
+    h->wait_view = -1;
     // decided once: the scratch below is that of the kernel that runs
     SolveKernel kernel = kSolveRows;
     bool captured = false;
@@ -1480,6 +1483,10 @@ static capsp_status_t enqueue_rows(capsp_handle_t h, int v, const T *b, T *x, in
             CAPSP_TRY(ensure_xp(h, nrhs));
         if (rv.late)
             CAPSP_TRY(launch_view_refresh(h, rv, h->d_err + 3, st));
+        if (kernel != kSolveStream) {  // which names the rows itself
+            h->wait_view = v;
+            h->wait_ring = kernel == kSolveChain ? rv.chain.ring : 0;
+        }
     }
     for (int r0 = 0; r0 < nrhs; r0 += 32) {
         const int nb = nrhs - r0 < 32 ? nrhs - r0 : 32;
@@ -1581,6 +1588,7 @@ static capsp_status_t enqueue_cols(capsp_handle_t h, const T *b, T *x, int nrhs,
 {
     CAPSP_TRY(ensure_column_scratch(h, nrhs));
     CAPSP_TRY(ensure_column_order(h, backward));
+    h->wait_view = -1;
     for (int r0 = 0; r0 < nrhs; r0 += 32) {
         const int nb = nrhs - r0 < 32 ? nrhs - r0 : 32;
         if (kPackedColumns) {
@@ -1780,6 +1788,30 @@ extern "C" capsp_status_t capsp_reserve(capsp_handle_t h, int max_nrhs)
     return CAPSP_OK;
 }
 
+// The rows of a reported wait.  On a level-ordered solve the row kernels name a row and
+// the position it waits on, the chain kernel a row or chain_code(its position), and a
+// position or chain_code(a place in its ring): the latest position before the row's, or
+// its own, that has this place.
+static void name_wait(capsp_handle_t h, int *row, int *on)
+{
+    if (h->wait_view < 0 || !h->view[h->wait_view].built)
+        return;
+    std::unique_ptr<int[]> perm(new (std::nothrow) int[(size_t)h->n]);
+    if (!perm || cudaMemcpy(perm.get(), h->view[h->wait_view].d_perm, sizeof(int) * (size_t)h->n,
+                            cudaMemcpyDeviceToHost) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (h->wait_ring > 0 && *row <= -2)
+        *row = perm[std::min(-2 - *row, h->n - 1)];
+    if (h->wait_ring > 0 && *on <= -2) {
+        const int p = (int)(std::find(perm.get(), perm.get() + h->n, *row) - perm.get());
+        *on = p - ((p - (-2 - *on)) & (h->wait_ring - 1));
+    }
+    if (*on >= 0)
+        *on = *on < h->n ? perm[*on] : -1;
+}
+
 extern "C" capsp_status_t capsp_status_sync(capsp_handle_t h, void *stream)
 {
     if (!h)
@@ -1788,11 +1820,13 @@ extern "C" capsp_status_t capsp_status_sync(capsp_handle_t h, void *stream)
     CAPSP_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     int err[4] = {0, 0, 0, 0};
     CAPSP_CUDA(cudaMemcpy(err, h->d_err, sizeof(err), cudaMemcpyDeviceToHost));
-    if (err[kErrStatus] == kStatusTimeout)
+    if (err[kErrStatus] == kStatusTimeout) {
+        name_wait(h, &err[kErrRow], &err[kErrWaitedOn]);
         return fail(CAPSP_ERR_TIMEOUT,
                     "dependency wait ran out of its budget (row/column %d waiting on %d); the "
                     "affected results are NaN",
                     err[kErrRow], err[kErrWaitedOn]);
+    }
     if (err[kErrStatus] != 0)
         return fail(CAPSP_ERR_CUDA, "device reported status %d", err[kErrStatus]);
     return CAPSP_OK;

@@ -175,11 +175,17 @@ __device__ __forceinline__ void ring_store(unsigned at, unsigned v)
 // the partner's own waits for values; two budgets of one wait are the
 // backstop.  True: the warp abandons its role (and so, in turn, do those that
 // wait for it).
+//
+// What gives up reports its position p as chain_code(p) where it has no row at hand,
+// and what it waits on as a position, or as chain_code(place in the ring); the host
+// names the rows (capsp_status_sync).
+__device__ __forceinline__ int chain_code(unsigned at) { return -2 - (int)at; }
+
 struct RoleWait {
     unsigned it;
     unsigned long long t0;
     __device__ __forceinline__ RoleWait() : it(0), t0(0) {}
-    __device__ __forceinline__ bool expired(const WaitCfg &w, int *err, int row)
+    __device__ __forceinline__ bool expired(const WaitCfg &w, int *err, int p)
     {
         if ((++it & 255u) != 0u)
             return false;
@@ -191,7 +197,7 @@ struct RoleWait {
         if (now - t0 <= 2ull * w.timeout_ns)
             return false;
         if (atomicCAS(err + kErrStatus, 0, kStatusTimeout) == 0) {
-            err[kErrRow] = row;
+            err[kErrRow] = chain_code(p);
             err[kErrWaitedOn] = -1;
         }
         return true;
@@ -207,7 +213,7 @@ __device__ __forceinline__ T chain_far_value(const ChainArgs<T> &a, const typena
     typedef VBits<T> VB;
     Spin sp;
     while (u == VB::kPending) {
-        if (sp.next(a.err, a.wait, p, q))
+        if (sp.next(a.err, a.wait, chain_code(p), q))
             return VB::from(VB::kQNaN);
         u = ld_relaxed(xp + q, pol);
     }
@@ -359,7 +365,7 @@ __device__ __forceinline__ void chain_feed(const ChainArgs<T> &a, unsigned base,
 #pragma unroll
                 for (int t = 0; t < 4; ++t)
                     if (k + 32 * t < he)
-                        part = fma(v[t], chain_far_value<T>(a, xp, q[t], u[t], p, keep), part);
+                        part = fma(v[t], chain_far_value<T>(a, xp, q[t], u[t], p - lane + l, keep), part);
             }
             __syncwarp();
 #pragma unroll
@@ -474,7 +480,7 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
                                 ++k;
                                 --left;
                             }
-                        } else if ((++polls & 15u) == 0u && sp.next(a.err, a.wait, row, (int)q)) {
+                        } else if ((++polls & 15u) == 0u && sp.next(a.err, a.wait, row, chain_code(q))) {
                             acc = VB::from(VB::kQNaN);
                             left = 0;
                             j0 = j1;
@@ -541,7 +547,7 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
                         }
                     }
                 }
-                if ((++polls & 255u) == 0u && left > 0 && sp.next(a.err, a.wait, row, (int)q0)) {
+                if ((++polls & 255u) == 0u && left > 0 && sp.next(a.err, a.wait, row, chain_code((q0 - ring_at) / (unsigned)sizeof(U)))) {
                     acc = VB::from(VB::kQNaN);
                     left = 0;
                     q0 = q1 = never;

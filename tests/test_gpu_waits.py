@@ -9,6 +9,7 @@ import pytest
 import capellinisptrsv_gb300 as cs
 import oracle
 from conftest import rel_inf_err
+from test_gpu_chain import dense
 from test_gpu_stream import blocks, dev, host
 
 torch = pytest.importorskip("torch")
@@ -43,3 +44,33 @@ def test_stream_reports_the_waiting_row(k):
     s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(m.val))
     b = np.random.default_rng(k).standard_normal((m.n, k))
     check(m, reported(m, s, b, stuck), stuck)
+
+
+CHAINS = {
+    # near entries only; far entries, folded by a lane or by a warp; entries walked in global memory
+    "near": lambda: cs.generate(n=1_025, kmin=1, kmax=6, band=60, seed=3),
+    "far": lambda: cs.generate("zipf40_1m", n=25_385, seed=7),
+    "far_light": lambda: cs.generate(n=60_000, kmin=6, kmax=12, band=9_000, seed=8),
+    "spilled": lambda: dense(700),
+}
+
+
+@pytest.mark.parametrize("k", [1, 3])
+@pytest.mark.parametrize("name", list(CHAINS))
+def test_chain_reports_the_waiting_row(name, k):
+    """Rows, not positions of the level order nor places in the ring."""
+    m = CHAINS[name]()
+    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(m.val))
+    rng = np.random.default_rng(k)
+    for stuck in (m.colidx[m.rowptr[m.n // 3]], m.colidx[m.rowptr[m.n - 3] + 1]):
+        check(m, reported(m, s, rng.standard_normal((m.n, k)), int(stuck)), int(stuck))
+
+
+@pytest.mark.parametrize("algorithm", ["wrtfst", "mix"])
+def test_row_kernels_report_rows(algorithm):
+    """Their waits, too, are named by row on the level schedule."""
+    m = blocks(12, 1_031, 3, 11, 14)
+    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(m.val))
+    s.set_algorithm(algorithm)
+    stuck = int(m.colidx[m.rowptr[2_000]])
+    check(m, reported(m, s, cs.normal(m.n, seed=14), stuck), stuck)

@@ -114,6 +114,7 @@ struct RowView {
     int upper = 0;        // its rows are upper-triangular (diagonal first)
     int levels = 0;
     int longest = 0;      // dependencies of its longest row
+    int heavy[3] = {0, 0, 0};  // rows in groups of 32, 16 and 8 that average kHeavyEntries stored entries
     bool narrow = false;  // levels narrower than ~4k rows on average
     int *d_perm = nullptr, *d_lptr = nullptr, *d_lidx = nullptr, *d_lsrc = nullptr, *d_dsrc = nullptr;
     void *d_lval = nullptr, *d_linv = nullptr;
@@ -514,6 +515,32 @@ static ChainPlan plan_chain(int n, int levels, size_t vb, const int *lptr, const
     return c;
 }
 
+// rows of a view's groups of group_rows that hold kHeavyEntries stored entries a row
+static int heavy_rows(int n, int group_rows, const int *lcum)
+{
+    long long rows = 0;
+    for (int p = 0; p < n; p += group_rows) {
+        const int e = std::min(n, p + group_rows);
+        if ((long long)lcum[e] - lcum[p] >= (long long)kHeavyEntries * (e - p))
+            rows += e - p;
+    }
+    return (int)rows;
+}
+
+// what auto_kernel() looks at, for `cols` right-hand sides (rounded up)
+static ViewShape view_shape(capsp_handle_t h, const RowView &rv, int cols)
+{
+    ViewShape s;
+    s.n = h->n;
+    s.levels = rv.levels;
+    s.entries = (long long)h->nnz - h->n;
+    s.longest = rv.longest;
+    s.heavy = cols < 8 ? rv.heavy[cols / 2] : 0;
+    s.chain = rv.chain.ok;
+    s.f64 = h->dtype == CAPSP_R_64F;
+    return s;
+}
+
 // Layout of the stream kernel for a view whose level layout is built
 // (rv.stream.ok, unless padding would double the entries); synchronous.
 static capsp_status_t build_stream(capsp_handle_t h, RowView &rv)
@@ -646,6 +673,8 @@ static capsp_status_t build_view(capsp_handle_t h, int v)
     rv.longest = 0;
     for (int k = 0; k < n; ++k)
         rv.longest = std::max(rv.longest, lptr[(size_t)k + 1] - lptr[(size_t)k]);
+    for (int g = 0; g < 3; ++g)
+        rv.heavy[g] = rv.longest + 1 >= kHeavyEntries ? heavy_rows(n, 32 >> g, rv.h_lcum.data()) : 0;
     rv.upper = upper;
     rv.levels = levels;
     std::vector<int> lnear;
@@ -675,7 +704,7 @@ static capsp_status_t build_view(capsp_handle_t h, int v)
         return fail(CAPSP_ERR_CUDA, "level-schedule upload failed");
     if (bad != INT_MAX)
         return fail(CAPSP_ERR_INVALID, "zero or non-finite diagonal at schedule position %d", bad);
-    if (rv.longest <= kStreamLongest && (long long)n >= kStreamAnyRows * (long long)levels)
+    if (auto_kernel(view_shape(h, rv, 1), 1) == kSolveStream)
         return build_stream(h, rv);
     return CAPSP_OK;
 }
@@ -834,7 +863,7 @@ extern "C" capsp_status_t capsp_batched_create(int nsys, const int *sys_rowoff, 
     // built here for wide ones, not inside the first such solve (264 systems of 2.8 M
     // rows, 4 RHS: that solve 1.78 ms with the row kernel, 2.33 ms when it built the layout)
     RowView &rv = h->view[0];
-    if (rv.built && rv.longest <= kStreamLongest && !rv.narrow) {
+    if (rv.built && !rv.narrow && auto_kernel(view_shape(h, rv, 4), 4) == kSolveStream) {
         DeviceGuard g(h->device);
         const capsp_status_t s = build_stream(h, rv);
         if (s != CAPSP_OK) {
@@ -1327,14 +1356,8 @@ static SolveKernel kernel_wanted(capsp_handle_t h, int v, const Tuning &tn, int 
     if (!view_level(h, v) || !rv.built || tn.kind >= 0 || !tn.dflt || h->border_explicit || h->row_kernels_only ||
         h->trace != nullptr || h->l2_mode != CAPSP_L2_HINTS)
         return kSolveRows;
-    ViewShape s;
-    s.n = h->n;
-    s.levels = rv.levels;
-    s.entries = (long long)h->nnz - h->n;
-    s.longest = rv.longest;
-    s.chain = rv.chain.ok;
-    s.f64 = h->dtype == CAPSP_R_64F;
-    return auto_kernel(s, lanes_for_rhs(nrhs < 32 ? nrhs : 32));
+    const int cols = lanes_for_rhs(nrhs < 32 ? nrhs : 32);
+    return auto_kernel(view_shape(h, rv, cols), cols);
 }
 
 // Where row `row` is in a stream layout (debug hook of a row that never publishes;

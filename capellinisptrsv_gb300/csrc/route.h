@@ -22,10 +22,20 @@ constexpr long long kStreamAnyRows = 12288;
 // time, so longer ones are for the mixed row kernel's warps.  (Banded matrices
 // have some of 40 to 110 entries in their transposes, where few columns precede.)
 constexpr int kStreamLongest = 128;
+// ... and the share of rows (1 / this) in groups that the mixed row kernel would give
+// a warp per row, with fewer than 8 right-hand sides.  A warp sums a row as a tree, a
+// lane one entry after the other; where such rows are the norm that shows (12,800 rows
+// per level, 33-60 entries, 2-norm of the error against more than 64 bits: FP64 2.6e-17,
+// in a lane 4.6e-17; FP32 1.4e-8, 2.4e-8), where they are few it is lost in the rest
+// (a seventh or a sixth of the rows: 1.02 to 1.06 times the error).  With 8 and more
+// the row kernels use a lane too.
+constexpr long long kStreamHeavyShare = 6;
+constexpr int kHeavyEntries = 32;  // stored entries per row of such a group, on average
 
 struct ViewShape {
     long long n = 0, levels = 0, entries = 0;  // rows, levels, off-diagonal entries
     int longest = 0;                           // off-diagonal entries of the longest row
+    long long heavy = 0;                       // rows in heavy groups, as grouped for `cols`
     bool chain = false;                        // a launch plan of the chain kernel exists
     bool f64 = true;
 };
@@ -51,7 +61,7 @@ inline SolveKernel auto_kernel(const ViewShape &s, int cols)
 {
     if (s.chain)
         return kSolveChain;
-    if (s.longest > kStreamLongest || s.levels < 1)
+    if (s.longest > kStreamLongest || s.levels < 1 || (cols < 8 && kStreamHeavyShare * s.heavy > s.n))
         return kSolveRows;
     const long long rows = s.n / s.levels;  // per level
     if (rows >= kStreamAnyRows)

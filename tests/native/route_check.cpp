@@ -55,6 +55,15 @@ int main()
     CHECK(auto_kernel(shape(4095, 3, 6, 12, true), 4) == kSolveStream);
     CHECK(auto_kernel(shape(300, 3, 4, 12, false), 4) == kSolveStream);
     CHECK(auto_kernel(shape(300, 3, 4, 12, false), 2) == kSolveRows);
+    // rows that the mixed row kernel would sum as trees: a few of them, or more, with
+    // fewer than 8 right-hand sides and with 8
+    for (int cols = 1; cols <= 32; cols *= 2) {
+        ViewShape s = shape(12800, 4, 40, 60, true);
+        s.heavy = s.n / 6;
+        CHECK(auto_kernel(s, cols) == kSolveStream);
+        s.heavy = s.n / 6 + 1;
+        CHECK(auto_kernel(s, cols) == (cols < 8 ? kSolveRows : kSolveStream));
+    }
     std::printf("routes ok\n");
     return 0;
 }

@@ -9,6 +9,7 @@ import pytest
 import capellinisptrsv_gb300 as cs
 import oracle
 from conftest import rel_inf_err
+from test_gpu_stream import blocks
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -81,4 +82,32 @@ def test_fp32_products_beyond_the_range_that_cancel():
     assert rel_inf_err(x, xo) <= 1e-5
     s.set_algorithm("wrtfst")
     assert rel_inf_err(host(s.solve(dev(b))), xo) <= 1e-5
+    s.status()
+
+
+def solve_longdouble(m, v, b):
+    """Forward solve in extended precision (128-bit, or at least 80-bit, floats)."""
+    v, x = v.astype(np.longdouble), b.astype(np.longdouble)
+    for i in range(m.n):
+        j0, j1 = m.rowptr[i], m.rowptr[i + 1] - 1
+        x[i] = (x[i] - np.dot(v[j0:j1], x[m.colidx[j0:j1]])) / v[j1]
+    return x
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("k", [1, 4])
+def test_long_rows_are_as_exact_as_in_the_mixed_kernel(k, dtype):
+    """Wide levels of 33 to 60 entries a row: the error is that of the mixed row kernel,
+    which sums a row as a tree (a hundredth more for the order of equal terms)."""
+    m = blocks(2, 12_800, 33, 60, 3)
+    v = m.val.astype(dtype)
+    b = np.random.default_rng(k).standard_normal((m.n, k)).astype(dtype)
+    xo = solve_longdouble(m, v, b)
+    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(v))
+    err = {}
+    for algorithm in ("auto", "mix"):
+        s.set_algorithm(algorithm)
+        d = host(s.solve(dev(b))).astype(np.longdouble) - xo
+        err[algorithm] = float(np.sqrt((d * d).sum() / (xo * xo).sum()))
+    assert err["auto"] <= 1.01 * err["mix"], err
     s.status()

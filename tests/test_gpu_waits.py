@@ -1,4 +1,4 @@
-"""Dependency waits that run out of their budget: what is reported, in every kernel."""
+"""Dependency waits that run out of their budget: what the stream and chain kernels report."""
 from __future__ import annotations
 
 import re
@@ -64,13 +64,3 @@ def test_chain_reports_the_waiting_row(name, k):
     rng = np.random.default_rng(k)
     for stuck in (m.colidx[m.rowptr[m.n // 3]], m.colidx[m.rowptr[m.n - 3] + 1]):
         check(m, reported(m, s, rng.standard_normal((m.n, k)), int(stuck)), int(stuck))
-
-
-@pytest.mark.parametrize("algorithm", ["wrtfst", "mix"])
-def test_row_kernels_report_rows(algorithm):
-    """Their waits, too, are named by row on the level schedule."""
-    m = blocks(12, 1_031, 3, 11, 14)
-    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(m.val))
-    s.set_algorithm(algorithm)
-    stuck = int(m.colidx[m.rowptr[2_000]])
-    check(m, reported(m, s, cs.normal(m.n, seed=14), stuck), stuck)

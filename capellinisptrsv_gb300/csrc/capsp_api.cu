@@ -87,6 +87,7 @@ typedef GraphCache<cudaGraphExec_t, destroy_graph_exec> Graphs;
 struct ChainPlan {
     bool ok = false;
     bool far = false;  // some entry reaches back beyond the ring
+    bool late = false; // a row's right-hand side joins its sum last
     int ring = 0, warps = 0, slots = 0, entries = 0, lag = 0, ahead = 0;
 };
 
@@ -455,7 +456,8 @@ constexpr int kChainFill = 131072;
 // dependencies per level: 146 us, 236 us with 8,192).  Half of a ring that wraps is the reach of near
 // entries; the other half lets the chain warps drift apart and marks positions
 // pending ahead of them.
-static ChainPlan plan_chain(int n, int levels, size_t vb, const int *lptr, const int *lidx, std::vector<int> &lnear)
+static ChainPlan plan_chain(int n, int levels, size_t vb, bool late, const int *lptr, const int *lidx,
+                            std::vector<int> &lnear)
 {
     ChainPlan c;
     if (!chain_levels(n, levels))
@@ -464,6 +466,7 @@ static ChainPlan plan_chain(int n, int levels, size_t vb, const int *lptr, const
     c.ring = 1024;
     while (c.ring < n && c.ring < (deep ? 16384 : 8192))
         c.ring *= 2;
+    c.late = late;
     const bool all = c.ring >= n;
     if (!all)
         c.ring = 4096;
@@ -478,13 +481,14 @@ static ChainPlan plan_chain(int n, int levels, size_t vb, const int *lptr, const
             chunk[(size_t)k] += lptr[q + 1] - lnear[(size_t)q];
     // the chain block holds words, ring and slots, a feeder words and a staging
     // area of a slot's size per warp
-    const int words = 1024 + 32, hdr = 32 * (int)(vb + 8);
+    const int words = 1024 + 32, hdr = chain_header_bytes((int)vb, late);
     const int shapes[4][2] = {{16, 4}, {16, 3}, {16, 2}, {8, 2}};  // warps, slots per warp
     long long large = 0;
     for (int k = deep ? 3 : 0; k < 4; ++k) {
         c.warps = shapes[k][0];
         c.slots = c.warps * shapes[k][1];
-        const int room = std::min((kChainSmem - words - c.ring * (int)vb) / c.slots, (kChainSmem - words) / kChainWarps);
+        const int room = std::min((kChainSmem - words - c.ring * (int)vb) / c.slots,
+                                  (kChainSmem - words) / kChainWarps - chain_base_bytes((int)vb, late));
         c.entries = (room - hdr) / (int)(vb + 2) / 8 * 8;
         large = std::count_if(chunk.begin(), chunk.end(), [&](int e) { return e > c.entries; });
         if (32 * large <= nchunks)
@@ -678,7 +682,9 @@ static capsp_status_t build_view(capsp_handle_t h, int v)
     rv.upper = upper;
     rv.levels = levels;
     std::vector<int> lnear;
-    rv.chain = plan_chain(n, levels, vb, lptr.data(), lidx.data(), lnear);
+    // where the row kernels give every row, or most, a warp (untuned) and sum it as a tree
+    const bool late = n < kDeepRows * levels || kStreamHeavyShare * rv.heavy[0] > n;
+    rv.chain = plan_chain(n, levels, vb, late, lptr.data(), lidx.data(), lnear);
     cudaFree(rv.d_lnear);
     rv.d_lnear = nullptr;
     if (rv.chain.ok) {
@@ -1237,7 +1243,7 @@ static Tuning untuned(capsp_handle_t h, Op op)
     // mixed at the reference's border of 10: 2.98 ms; one lane per row:
     // 1.96 ms).
     if ((h->alg == CAPSP_ALG_AUTO || h->alg == CAPSP_ALG_SYNCFREE_CSC) && !h->border_explicit) {
-        if (rv.built && view_level(h, v) && (long long)h->n < 32LL * (long long)rv.levels)
+        if (rv.built && view_level(h, v) && (long long)h->n < kDeepRows * (long long)rv.levels)
             t.border = 1;
         else if (t.border < 32)
             t.border = 32;
@@ -1463,6 +1469,7 @@ static capsp_status_t enqueue_chain(capsp_handle_t h, int v, const T *b, T *x, i
     a.entries = cp.entries;
     a.lag = cp.lag;
     a.ahead = cp.ahead;
+    a.late = cp.late;
     a.fill = fill;
     a.reset_err = (!cp.far || fill) && first && nb == 1;
     a.err = h->d_err;
@@ -1972,7 +1979,8 @@ extern "C" capsp_status_t capsp_solve_host(capsp_handle_t h, const void *b_host,
         // with 4 right-hand sides, 32 bytes per read, 8.97 ms in place, 11.2
         // copied).
         void *b_in_place =
-            (!column_driven(h, kOpSolve) && view_level(h, v) && !(wide_levels(h, v) && nrhs == 1))
+            (!column_driven(h, kOpSolve) && view_level(h, v) && !(wide_levels(h, v) && nrhs == 1) &&
+             !(chain && h->view[v].chain.late && h->dtype == CAPSP_R_64F))  // reads b per entry
                 ? pinned_alias(b_host, h->device)
                 : nullptr;
         if (b_in_place && !chain) {

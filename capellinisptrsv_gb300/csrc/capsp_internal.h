@@ -71,6 +71,25 @@ struct RowArgs {
 constexpr int kChainWarps = 16;
 constexpr int kChainSmem = 232448;  // shared memory a block may take (227 KB)
 
+// bytes of a slot before its entries (kernels_chain.cuh)
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr int chain_header_bytes(int value_bytes, bool late)
+{
+    return 32 * (value_bytes + 8 + (late ? 2 * value_bytes : 0));
+}
+
+// bytes that a feeder warp needs beside a slot's (kernels_chain.cuh: chain_split)
+constexpr int kChainTile = 256;
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr int chain_base_bytes(int value_bytes, bool late)
+{
+    return late && value_bytes == 8 ? kChainTile * value_bytes : 0;
+}
+
 // Arguments of the chain solve: the level schedule (as RowArgs) and, per
 // position, lnear[p] = the first entry within reach of the ring of recent
 // values in shared memory (the entries before it are far: folded by the
@@ -96,6 +115,7 @@ struct ChainArgs {
     int entries;  // near entries a slot holds (a multiple of 8)
     int lag;      // chunks that the warps may drift apart (0: the ring holds the whole solve)
     int ahead;    // chunks ahead of its own that a warp marks pending
+    int late;     // the right-hand side joins a row's sum last (kernels_chain.cuh: LATE)
     int fill;     // mark the publication vector pending before the solve
     int reset_err;
     int *err;

@@ -59,16 +59,12 @@ constexpr unsigned kChainFreed = 576;    // per feeder warp: latest use its slot
 constexpr unsigned kChainRing = 1024;    // ring of values, or a feeder's staging
 
 // A slot: 32 partial sums, rows, and (offset | count << 16) words of the near
-// entries, then the entries' values and their ring indices.
-template <typename T>
-__host__ __device__ constexpr unsigned chain_header_bytes()
-{
-    return 32u * (unsigned)(sizeof(T) + 8);
-}
-template <typename T>
+// entries (LATE: and right-hand sides and 1/diagonals), then the entries' values and
+// their ring indices.
+template <typename T, bool LATE>
 __host__ __device__ constexpr unsigned chain_slot_bytes(int entries)
 {
-    return chain_header_bytes<T>() + (unsigned)entries * (unsigned)(sizeof(T) + 2);
+    return (unsigned)chain_header_bytes(sizeof(T), LATE) + (unsigned)entries * (unsigned)(sizeof(T) + 2);
 }
 
 __device__ __forceinline__ unsigned cluster_ctarank()
@@ -239,8 +235,48 @@ __device__ __forceinline__ float chain_sum(float acc, float low)
     return fabsf(sum) <= 3.402823466e38f ? sum : acc;
 }
 
-// Feeder: chunks c = s, s + step, ... of one slot.
+// LATE, for matrices whose rows the row kernels sum a warp at a time: a row's entries
+// are summed from zero and its right-hand side joins last, as there, so that the value
+// takes one rounding of its own size, not one per entry.  2-norm of the error against
+// more than 64 bits, with the right-hand side first / LATE / row kernel: FP64 3.0e-16 /
+// 8.4e-17 / 6.8e-17 (131,072 rows of 40 dependencies), 9.2e-17 / 7.8e-17 / 7.6e-17
+// (200,000 Zipf rows), 1.36e-16 / 8.9e-17 / 8.1e-17 (2,003 rows of 3-12); FP32 5.0e-8 /
+// 3.5e-8 / 3.7e-8, 4.9e-8 / 4.0e-8 / 4.1e-8, 4.6e-8 / 3.9e-8 / 4.1e-8.
+//
+// In single precision that is an FMA at the row's end (200,000 Zipf rows 3.36 -> 3.39
+// ms).  An FP64 one there would hold up every link (1,048,576 Zipf rows 28.3 -> 37.6
+// ms), so there the chain carries s = x - b/d: a row's s is the sum of v x over its far
+// entries and of v b/d over its near ones, both known to the feeders ahead of time, and
+// of v s over the near ones, in the chain.  x = b/d + s is formed off the chain, where it
+// is stored (28.4 ms; the 2,003 rows 27.6 -> 29.0 us).
+template <typename T, bool LATE>
+__host__ __device__ constexpr bool chain_split()
+{
+    return LATE && sizeof(T) == 8;
+}
+
+// what a row hands to the chain, and the value of x
+template <typename T, bool LATE>
+__device__ __forceinline__ T chain_link(T acc, T low, T bv, T dinv)
+{
+    const T sum = chain_sum(acc, low);
+    return LATE && !chain_split<T, LATE>() ? fma(bv, dinv, sum) : sum;
+}
+template <typename T, bool LATE>
+__device__ __forceinline__ T chain_x(T link, T bv, T dinv)
+{
+    return chain_split<T, LATE>() ? fma(bv, dinv, link) : link;
+}
+
+// b/d of position q
 template <typename T>
+__device__ __forceinline__ T chain_base(const ChainArgs<T> &a, const T *b, int q)
+{
+    return __ldg(b + (size_t)__ldg(a.perm + q) * (size_t)a.ld) * __ldg(a.linv + q);
+}
+
+// Feeder: chunks c = s, s + step, ... of one slot.
+template <typename T, bool LATE>
 __device__ __forceinline__ void chain_feed(const ChainArgs<T> &a, unsigned base, unsigned char *smem, int rank,
                                            int warp, int lane, const T *b, const T *xp_r)
 {
@@ -251,12 +287,14 @@ __device__ __forceinline__ void chain_feed(const ChainArgs<T> &a, unsigned base,
     if (g >= per_slot * a.slots)
         return;
     const int s = g % a.slots;
-    const unsigned slot_bytes = chain_slot_bytes<T>(a.entries);
-    const unsigned hdr = chain_header_bytes<T>();
-    unsigned char *mine = smem + kChainRing + (size_t)warp * slot_bytes;
+    const unsigned slot_bytes = chain_slot_bytes<T, LATE>(a.entries);
+    const unsigned hdr = (unsigned)chain_header_bytes(sizeof(T), LATE);
+    unsigned char *mine = smem + kChainRing + (size_t)warp * (slot_bytes + chain_base_bytes(sizeof(T), LATE));
     T *m_acc = reinterpret_cast<T *>(mine);
     int *m_row = reinterpret_cast<int *>(mine + 32 * sizeof(T));
     unsigned *m_meta = reinterpret_cast<unsigned *>(m_row + 32);
+    T *m_late = reinterpret_cast<T *>(m_meta + 32);
+    T *m_base = reinterpret_cast<T *>(mine + slot_bytes);  // chain_split: b/d of a tile of entries
     T *m_val = reinterpret_cast<T *>(mine + hdr);
     unsigned short *m_idx = reinterpret_cast<unsigned short *>(m_val + a.entries);
     const unsigned dst = cluster_map(base + kChainRing + (unsigned)a.ring * (unsigned)sizeof(U) + 16u + (unsigned)s * slot_bytes, 0);
@@ -278,7 +316,13 @@ __device__ __forceinline__ void chain_feed(const ChainArgs<T> &a, unsigned base,
             fs = ld_stream(a.lptr + p, stream);
             ns = ld_stream(a.lnear + p, stream);
             ne = ld_stream(a.lptr + p + 1, stream);
-            acc = ld_stream(b + (size_t)row * (size_t)a.ld, stream) * ld_stream(a.linv + p, stream);
+            const T bv = ld_stream(b + (size_t)row * (size_t)a.ld, stream), dinv = ld_stream(a.linv + p, stream);
+            if (LATE) {
+                m_late[lane] = bv;
+                m_late[32 + lane] = dinv;
+            } else {
+                acc = bv * dinv;
+            }
         }
         // near entries: one after another in the slot, rows that do not fit are
         // left to the chain block (it then reads them from global memory)
@@ -296,6 +340,7 @@ __device__ __forceinline__ void chain_feed(const ChainArgs<T> &a, unsigned base,
         const int total = __reduce_min_sync(kFullMask, spill ? off : whole);
         m_row[lane] = row;
         m_meta[lane] = spill && cnt > 0 ? kChainSpill : ((unsigned)off & 0xffffu) | ((unsigned)cnt << 16);
+        constexpr bool split = chain_split<T, LATE>();
         for (int k0 = 0; k0 < total; k0 += 128) {
             int src[4];
 #pragma unroll
@@ -319,6 +364,38 @@ __device__ __forceinline__ void chain_feed(const ChainArgs<T> &a, unsigned base,
                     m_idx[k] = (unsigned short)((unsigned)qi[t] & mask);
                     m_val[k] = qv[t];
                 }
+            }
+            if constexpr (split) {
+                T base[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    base[t] = k0 + 32 * t + lane < total ? chain_base(a, b, qi[t]) : T(0);
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    m_base[(k0 + 32 * t + lane) % kChainTile] = base[t];
+                // a tile is there: each lane takes its row's part of it
+                const int tile = k0 / kChainTile * kChainTile;
+                if (k0 + 128 - tile == kChainTile || k0 + 128 >= total) {
+                    __syncwarp();
+                    const int k1 = spill ? 0 : min(min(off + cnt, total), tile + kChainTile);
+                    for (int k = max(off, tile); k < k1; ++k)
+                        acc = fma(m_val[k], m_base[k - tile], acc);
+                    __syncwarp();
+                }
+            }
+        }
+        if constexpr (split) {
+            for (int k = spill ? ns : ne; k < ne; k += 4) {
+                T v[4], base[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    v[t] = k + t < ne ? ld_stream(a.lval + k + t, stream) : T(0);
+                    base[t] = k + t < ne ? chain_base(a, b, ld_stream(a.lidx + k + t, stream)) : T(0);
+                }
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    if (k + t < ne)
+                        acc = fma(v[t], base[t], acc);
             }
         }
         // far dependencies of light rows: one row per lane, eight loads in flight
@@ -401,13 +478,13 @@ __device__ __forceinline__ void chain_feed(const ChainArgs<T> &a, unsigned base,
 }
 
 // Chain block: chunks c = warp, warp + W, ...
-template <typename T>
+template <typename T, bool LATE>
 __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base, unsigned char *smem, int warp,
                                            int lane, T *x, T *xp_r)
 {
     typedef VBits<T> VB;
     typedef typename VB::U U;
-    const unsigned slot_bytes = chain_slot_bytes<T>(a.entries);
+    const unsigned slot_bytes = chain_slot_bytes<T, LATE>(a.entries);
     const unsigned ring_at = base + kChainRing, never = ring_at + (unsigned)a.ring * (unsigned)sizeof(U);
     unsigned char *slots = smem + kChainRing + (size_t)a.ring * sizeof(U) + 16;
     volatile int *done = reinterpret_cast<volatile int *>(smem + kChainDone);
@@ -441,12 +518,14 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
         }
         const unsigned char *slot = slots + (size_t)s * slot_bytes;
         const unsigned slot_at = never + 16u + (unsigned)s * slot_bytes;
-        const T *s_val = reinterpret_cast<const T *>(slot + chain_header_bytes<T>());
+        const T *s_val = reinterpret_cast<const T *>(slot + (unsigned)chain_header_bytes(sizeof(T), LATE));
         const unsigned short *s_idx = reinterpret_cast<const unsigned short *>(s_val + a.entries);
         bool open = p < a.n;
         T acc = reinterpret_cast<const T *>(slot)[lane], low = T(0);
         const int row = reinterpret_cast<const int *>(slot + 32 * sizeof(T))[lane];
         const unsigned meta = reinterpret_cast<const unsigned *>(slot + 32 * sizeof(T) + 128)[lane];
+        const T *late = reinterpret_cast<const T *>(slot + 32 * sizeof(T) + 256);
+        const T bv = LATE && open ? late[lane] : T(0), dinv = LATE && open ? late[32 + lane] : T(0);
         int k = (int)(meta & 0xffffu), left = open && meta != kChainSpill ? (int)(meta >> 16) : 0;
         // a row that must not publish (debug) waits for itself
         const bool stuck = open && row == a.stuck_row;
@@ -488,15 +567,18 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
                         }
                     }
                     if (j0 >= j1 && left == 0 && !wait_own) {
-                        acc = chain_sum(acc, low);
+                        acc = chain_link<T, LATE>(acc, low, bv, dinv);
                         ring_store(own, VB::to(acc));
                         open = false;
                     }
                 }
             }
         } else {
-            if (open && left == 0)
+            if (open && left == 0) {
+                if (LATE)
+                    acc = chain_link<T, LATE>(acc, low, bv, dinv);
                 ring_store(own, VB::to(acc));
+            }
             // Every round loads, side by side, the ring value of the row's next
             // dependency, that entry's value and the next entry's index; a lane
             // that is done polls the word after the ring, which stays pending.
@@ -506,8 +588,8 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
             // of 40 dependencies 26 % slower).
             constexpr bool two = sizeof(T) == 4;
             unsigned q0 = never, q1 = never;
-            unsigned at_v = slot_at + chain_header_bytes<T>() + (unsigned)sizeof(T) * (unsigned)k;
-            unsigned at_i = slot_at + chain_header_bytes<T>() + (unsigned)sizeof(T) * (unsigned)a.entries + 2u * (unsigned)k;
+            unsigned at_v = slot_at + (unsigned)chain_header_bytes(sizeof(T), LATE) + (unsigned)sizeof(T) * (unsigned)k;
+            unsigned at_i = slot_at + (unsigned)chain_header_bytes(sizeof(T), LATE) + (unsigned)sizeof(T) * (unsigned)a.entries + 2u * (unsigned)k;
             if (left > 0)
                 q0 = ring_at + (unsigned)sizeof(U) * shared_u16(at_i);
             if (two && left > 1)
@@ -541,7 +623,7 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
                         if (two && left < 2)
                             q1 = never;
                         if (left == 0) {
-                            acc = chain_sum(acc, low);
+                            acc = chain_link<T, LATE>(acc, low, bv, dinv);
                             ring_store(own, VB::to(acc));
                             q0 = never;
                         }
@@ -561,9 +643,10 @@ __device__ __forceinline__ void chain_walk(const ChainArgs<T> &a, unsigned base,
             done[warp] = c + a.warps;
         // the caller's x and the publication vector: off the chain
         if (p < a.n && !stuck) {
+            const T out = chain_x<T, LATE>(acc, bv, dinv);
             if (xp != nullptr)
-                st_relaxed(xp + p, VB::to(acc), keep);
-            st_stream(reinterpret_cast<U *>(x) + (size_t)row * (size_t)a.ld, VB::to(acc), stream);
+                st_relaxed(xp + p, VB::to(out), keep);
+            st_stream(reinterpret_cast<U *>(x) + (size_t)row * (size_t)a.ld, VB::to(out), stream);
         }
         __syncwarp();
     }
@@ -600,7 +683,7 @@ __device__ __forceinline__ void chain_usher(const ChainArgs<T> &a, unsigned base
     }
 }
 
-template <typename T>
+template <typename T, bool LATE>
 __global__ void __launch_bounds__(kChainThreads, 1) chain_solve_kernel(const ChainArgs<T> a)
 {
     typedef VBits<T> VB;
@@ -634,24 +717,26 @@ __global__ void __launch_bounds__(kChainThreads, 1) chain_solve_kernel(const Cha
     cluster_sync_all();
     if (rank != 0) {
         if (warp < kChainWarps)
-            chain_feed<T>(a, base, chain_smem, rank, warp, lane, a.b + rhs, xp);
+            chain_feed<T, LATE>(a, base, chain_smem, rank, warp, lane, a.b + rhs, xp);
     } else if (warp == kChainWarps)
         chain_usher<T>(a, base, chain_smem, lane);
     else if (warp < a.warps)
-        chain_walk<T>(a, base, chain_smem, warp, lane, a.x + rhs, xp);
+        chain_walk<T, LATE>(a, base, chain_smem, warp, lane, a.x + rhs, xp);
     // no block leaves while another may still write to its shared memory
     __syncwarp();
     cluster_sync_all();
 }
 
-template <typename T>
-cudaError_t launch_chain_solve(const ChainArgs<T> &a, int nrhs, cudaStream_t st)
+template <typename T, bool LATE>
+static cudaError_t launch_chain(const ChainArgs<T> &a, int nrhs, cudaStream_t st)
 {
-    const size_t staged = (size_t)kChainWarps * chain_slot_bytes<T>(a.entries);
-    const size_t chain = (size_t)a.ring * sizeof(T) + 16 + (size_t)a.slots * chain_slot_bytes<T>(a.entries);
+    const size_t staged =
+        (size_t)kChainWarps * (chain_slot_bytes<T, LATE>(a.entries) + (size_t)chain_base_bytes(sizeof(T), LATE));
+    const size_t chain = (size_t)a.ring * sizeof(T) + 16 + (size_t)a.slots * chain_slot_bytes<T, LATE>(a.entries);
     const size_t smem = kChainRing + (staged > chain ? staged : chain) + 16;  // the last slot's look-ahead
     // the limit is the kernel's, not the launch's: one value for all handles and threads
-    cudaError_t e = cudaFuncSetAttribute(chain_solve_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kChainSmem);
+    cudaError_t e = cudaFuncSetAttribute(chain_solve_kernel<T, LATE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         kChainSmem);
     if (e != cudaSuccess)
         return e;
     cudaLaunchAttribute at = {};
@@ -665,7 +750,13 @@ cudaError_t launch_chain_solve(const ChainArgs<T> &a, int nrhs, cudaStream_t st)
     cfg.stream = st;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, chain_solve_kernel<T>, a);
+    return cudaLaunchKernelEx(&cfg, chain_solve_kernel<T, LATE>, a);
+}
+
+template <typename T>
+cudaError_t launch_chain_solve(const ChainArgs<T> &a, int nrhs, cudaStream_t st)
+{
+    return a.late ? launch_chain<T, true>(a, nrhs, st) : launch_chain<T, false>(a, nrhs, st);
 }
 
 }  // namespace capsp

@@ -15,6 +15,9 @@ enum SolveKernel { kSolveRows = 0, kSolveChain = 1, kSolveStream = 2 };
 // against 147 us.
 constexpr long long kChainLevelRows = 256;
 
+// Rows per level below which the row kernels give every row a warp
+constexpr long long kDeepRows = 32;
+
 // Rows per level from which the stream kernel is the faster one whatever the
 // number of right-hand sides (auto_kernel)
 constexpr long long kStreamAnyRows = 12288;

@@ -111,3 +111,36 @@ def test_long_rows_are_as_exact_as_in_the_mixed_kernel(k, dtype):
         err[algorithm] = float(np.sqrt((d * d).sum() / (xo * xo).sum()))
     assert err["auto"] <= 1.01 * err["mix"], err
     s.status()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("kind", ["zipf40", "band", "deep_band"])
+def test_deep_matrices_are_solved_to_half_a_unit_in_the_last_place(kind, dtype):
+    """The 2-norm of the error is below that of half a unit in the last place of every
+    value: long rows do not add a rounding per entry."""
+    m = {"zipf40": lambda: cs.generate("zipf40_1m", n=20_001, seed=3),
+         "band": lambda: cs.generate(n=2_003, kmin=3, kmax=12, band=250, seed=3),
+         "deep_band": lambda: cs.generate(n=20_000, kmin=3, kmax=9, band=60, seed=3)}[kind]()
+    v = m.val.astype(dtype)
+    b = np.random.default_rng(1).standard_normal(m.n).astype(dtype)
+    xo = solve_longdouble(m, v, b)
+    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(v))
+    d = host(s.solve(dev(b))).astype(np.longdouble) - xo
+    assert float(np.sqrt((d * d).sum() / (xo * xo).sum())) <= np.finfo(dtype).eps / 2
+    s.status()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_nonfinite_right_hand_sides_in_deep_matrices(dtype):
+    """An infinity and a NaN in b reach the rows that they reach in the oracle, no others."""
+    m = cs.generate("zipf_1m", n=9_001, seed=5)
+    v = m.val.astype(dtype)
+    b = np.random.default_rng(5).standard_normal(m.n).astype(dtype)
+    b[8_000], b[8_500] = np.inf, np.nan
+    xo = oracle.solve_csr_lower(m.rowptr, m.colidx, v, b)
+    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(v))
+    x = host(s.solve(dev(b)))
+    ok = np.isfinite(xo)
+    assert 8_000 < ok.sum() < m.n - 2 and np.array_equal(np.isfinite(x), ok)
+    assert rel_inf_err(x[ok], xo[ok]) <= TOL[dtype]
+    s.status()

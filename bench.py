@@ -401,10 +401,8 @@ def run_native(args):
     peak, peak_kind = peaks()
     achieved = alg_bytes / (kms * 1e-3) / 1e9
     info = solver.info()
-    # "auto" solves levels of up to 256 rows with the chain kernel: one launch, and a
-    # fill where dependencies of a long solve reach beyond its ring (not counted in gpu_launches)
-    chain = m.n <= 256 * info["levels"]
-    kernel = "chain_solve" if chain else "row_solve"
+    ran = solver.last_solve()
+    kernel = ran["kernel"] + "_solve"
     traffic = profile_traffic(kernel, args.workload + "_" + args.dtype)
     # dependency-chain floor: a solve of L levels takes at least L - 1 hops,
     # each costing at least one publication's detection on another warp
@@ -441,7 +439,7 @@ def run_native(args):
             "cpu_baseline": cpu,
             "e2e": e2e,
             "cusparse_spsv": vendor,
-            "gpu_launches": (1 if chain else 2) * args.steps,
+            "gpu_launches": ran["launches"] * args.steps,
             "gflops_2nnz": world * 2.0 * m.nnz / (ms * 1e-3) / 1e9,
             "gbs_algorithmic": alg_bytes / (ms * 1e-3) / 1e9,
             "rel_err_vs_cpu_reference": rel, "max_abs_x_minus_ones": max_dev,
@@ -675,6 +673,7 @@ def measure_batched(args, ks, cpu_seconds, e2e: bool = True):
         batch.set_profiling(False)
         kms = statistics.mean(kms)
         info = batch.info()
+        ran = batch.last_solve()  # the autotuner may have preferred a launch shape of the row kernel
 
         # loop arm: a bounded, evenly spaced sample of systems, every RHS column
         nloop = max(1, min(nsys, LOOP_SOLVES_PER_STEP // k))
@@ -720,13 +719,12 @@ def measure_batched(args, ks, cpu_seconds, e2e: bool = True):
             "loop_systems": len(picks), "loop_ms_per_step": loop_ms,
             "rows_per_thread": info["rows_per_thread"], "block": info["block_threads"],
             "blocks_per_sm": info["blocks_per_sm"], "autotune_best_ms": tune_ms,
-            "loop_vs_batched_rel_err": worst, "clocks": clk.summary(),
+            "loop_vs_batched_rel_err": worst, "launches": ran["launches"], "clocks": clk.summary(),
         }
         entry["speedup_vs_loop"] = entry["solves_per_s"] / entry["loop_solves_per_s"]
         alg = algorithmic_bytes(m.n, m.nnz, 8, k)
         # DRAM bytes per launch from a committed capture of this k (default batch)
-        # (the stream kernel, unless the autotuner preferred a launch shape of the row kernel)
-        kernel = "stream_solve" if info["blocks_per_sm"] == 0 else "row_solve"
+        kernel = ran["kernel"] + "_solve"
         traffic = profile_traffic(kernel, f"batched_k{k}_f64") if nsys == BATCH_NSYS else None
         entry["roofline"] = {"bound": "hbm", "achieved": alg / (kms * 1e-3) / 1e9, "peak": peak, "unit": "GB/s",
                              "frac": alg / (kms * 1e-3) / 1e9 / peak, "traffic": traffic, "peak_kind": peak_kind,
@@ -788,7 +786,7 @@ def run_batched(args):
                          "no flush",
                    "parallelism": "single GPU"},
         "roofline": head["roofline"], "cpu_baseline": d["cpu_baseline"], "e2e": d["e2e"],
-        "gpu_launches": 2 * args.steps,
+        "gpu_launches": head["launches"] * args.steps,
         "loop_baseline": {"value": head["loop_solves_per_s"], "unit": "solves/s",
                           "what": "one single-RHS capsp_solve per system and RHS column, each system on its own "
                                   "handle, on an evenly spaced sample of systems"},
@@ -850,10 +848,10 @@ def measure_autograd(args, cpu_seconds):
     # grad_val pass (CUDA events on the launching stream around it alone)
     solver.set_profiling(True)
     x = solver.solve(b.detach())
-    kf = solver.last_kernel_ms()
+    kf, ran_f = solver.last_kernel_ms(), solver.last_solve()
     gx = (x - xstar).contiguous()
     y = solver.solve_transpose(gx)
-    kt = solver.last_kernel_ms()
+    kt, ran_t = solver.last_kernel_ms(), solver.last_solve()
     solver.set_profiling(False)
     gv_out = torch.empty(m.nnz, dtype=torch.float64, device=dev)
     solver.grad_val(y, x, out=gv_out)
@@ -918,15 +916,15 @@ def measure_autograd(args, cpu_seconds):
     peak, peak_kind = peaks()
     fwd_bytes = algorithmic_bytes(n, m.nnz, 8, k)
     grad_bytes = _grad_bytes(n, m.nnz, 8, k)
-    solve = "stream_solve" if k >= 4 else "row_solve"  # the kernel that "auto" takes
+    solve_f, solve_t = ran_f["kernel"] + "_solve", ran_t["kernel"] + "_solve"
     kernels = {
-        "forward_row_solve": {"kernel": solve + "_kernel", "kernel_ms": kf, "algorithmic_bytes_per_launch": fwd_bytes,
+        "forward_row_solve": {"kernel": solve_f + "_kernel", "kernel_ms": kf, "algorithmic_bytes_per_launch": fwd_bytes,
                               "achieved": fwd_bytes / (kf * 1e-3) / 1e9,
-                              "traffic": profile_traffic(solve, f"grad_1m_{k}rhs_f64")},
-        "transpose_row_solve": {"kernel": solve + "_kernel over the transposed view", "kernel_ms": kt,
+                              "traffic": profile_traffic(solve_f, f"grad_1m_{k}rhs_f64")},
+        "transpose_row_solve": {"kernel": solve_t + "_kernel over the transposed view", "kernel_ms": kt,
                                 "algorithmic_bytes_per_launch": fwd_bytes,
                                 "achieved": fwd_bytes / (kt * 1e-3) / 1e9,
-                                "traffic": profile_traffic(solve + "_transpose", f"grad_1m_{k}rhs_f64")},
+                                "traffic": profile_traffic(solve_t + "_transpose", f"grad_1m_{k}rhs_f64")},
         "grad_val": {"kernel": "grad_val_kernel", "kernel_ms": kg, "algorithmic_bytes_per_launch": grad_bytes,
                      "achieved": grad_bytes / (kg * 1e-3) / 1e9,
                      "fp64_fma_per_launch": float(m.nnz) * k,
@@ -944,10 +942,9 @@ def measure_autograd(args, cpu_seconds):
                                      "(upper CSR) + one grad_val pass"},
            "speedup_vs_loop": loop_ms / ms, "loop_vs_autograd_rel_err": agree, "clocks": clk.summary(),
            "e2e": {"value": e2e_ms, "unit": "ms", "h2d_bytes_per_step": int(2 * n * k * 8), "d2h_bytes_per_step": 8},
-           # forward: 1/diag + the level values of both views (3), pending
-           # fill, row solve; backward: pending fill, row solve over the
-           # transposed view, grad_val (no refresh: the values are still bound)
-           "gpu_launches_per_step": 8}
+           # forward: 1/diag + the level values of both views (3), the solve; backward: the
+           # solve over the transposed view, grad_val (no refresh: the values are still bound)
+           "gpu_launches_per_step": 3 + ran_f["launches"] + ran_t["launches"] + 1}
     out["cpu_baseline"] = None
     if cpu_seconds > 0:
         cpu, (xc, yc, gc) = _cpu_autograd(m, b_h, xs_h, cpu_seconds)

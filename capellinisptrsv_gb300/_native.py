@@ -32,6 +32,10 @@ class CapspError(RuntimeError):
         self.status = status
 
 
+class SolveReport(C.Structure):
+    _fields_ = [("kernel", C.c_int), ("launches", C.c_int), ("ring", C.c_int), ("far_entries", C.c_int)]
+
+
 class Info(C.Structure):
     _fields_ = [("n", C.c_int), ("nnz", C.c_int), ("dtype", C.c_int), ("format", C.c_int),
                 ("uplo", C.c_int), ("algorithm", C.c_int), ("mix_len", C.c_int),
@@ -73,6 +77,7 @@ _SIGS = {
     "capsp_set_backoff": (I, [H, C.c_uint]),
     "capsp_destroy": (I, [H]),
     "capsp_get_info": (I, [H, C.POINTER(Info)]),
+    "capsp_last_solve": (I, [H, C.POINTER(SolveReport)]),
     "capsp_set_algorithm": (I, [H, I]),
     "capsp_set_l2_policy": (I, [H, I]),
     "capsp_set_mix_border": (I, [H, I]),

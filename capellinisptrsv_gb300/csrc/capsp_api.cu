@@ -122,6 +122,7 @@ struct RowView {
     int *d_lnear = nullptr;   // first near entry per position (chain.ok only)
     ChainPlan chain;
     StreamPlan stream;
+    MixTable mix_info;  // capsp_get_info: the selector table's figures where no launch has needed it
     bool late = false;  // built after a refresh was captured: its values are refreshed before every solve
     std::vector<int> h_levels;  // first position of every level, and n
     std::vector<int> h_lcum;  // lptr[k] + k: row-count prefix in position space (mix tables)
@@ -215,6 +216,7 @@ struct capsp_handle_s {
     // (kMaxRetired: from then on scratch grows by powers of two up to 32).
     static constexpr int kMaxRetired = 24;
     bool solve_captured = false;
+    capsp_solve_report_t report = {};
     int wait_view = -1;  // view of the latest level-ordered solve (-1: another kind), whose waits ...
     int wait_ring = 0;   // ... name positions (row kernels: 0) or chain_code()s (chain kernel: its ring)
     bool own_capture = false;  // capsp_graph_solve's: its graphs are dropped when scratch changes
@@ -1425,6 +1427,7 @@ static capsp_status_t enqueue_stream(capsp_handle_t h, int v, const T *b, T *x, 
     // with 16; 16 RHS 1,100, 1,004 and 1,050 us; 750 rows, 16 RHS: 513 and 433 us)
     const int warps = per_level * cols < 10240 ? 8 : per_level * cols < 20480 ? 12 : 32;
     CAPSP_CUDA(launch_stream_solve<T>(a, long_rows, pairs, warps, h->num_sms, st));
+    h->report.launches += 2;
     if (prof)
         CAPSP_CUDA(cudaEventRecord(h->ev_k1, st));
     if (stuck_pos >= 0)
@@ -1445,8 +1448,10 @@ static capsp_status_t enqueue_chain(capsp_handle_t h, int v, const T *b, T *x, i
     // all-pending: a single right-hand side marks a short one itself, and needs
     // one launch, as it does without far dependencies
     const bool fill = cp.far && first && nb == 1 && h->n <= kChainFill;
-    if (cp.far && !fill)
+    if (cp.far && !fill) {
         CAPSP_CUDA(launch_fill_pending<T>((T *)h->d_xp, h->n, nb, nb, h->d_ticket, 1, first ? h->d_err : nullptr, st));
+        h->report.launches++;
+    }
     else if (first && nb > 1)
         CAPSP_CUDA(cudaMemsetAsync(h->d_err, 0, sizeof(int) * 4, st));
     ChainArgs<T> a;
@@ -1479,6 +1484,7 @@ static capsp_status_t enqueue_chain(capsp_handle_t h, int v, const T *b, T *x, i
     if (prof)
         CAPSP_CUDA(cudaEventRecord(h->ev_k0, st));
     CAPSP_CUDA(launch_chain_solve<T>(a, nb, st));
+    h->report.launches++;
     if (prof)
         CAPSP_CUDA(cudaEventRecord(h->ev_k1, st));
     return CAPSP_OK;
@@ -1511,12 +1517,21 @@ static capsp_status_t enqueue_rows(capsp_handle_t h, int v, const T *b, T *x, in
         }
         if (kernel != kSolveStream)
             CAPSP_TRY(ensure_xp(h, nrhs));
-        if (rv.late)
+        if (rv.late) {
             CAPSP_TRY(launch_view_refresh(h, rv, h->d_err + 3, st));
+            h->report.launches++;
+        }
         if (kernel != kSolveStream) {  // which names the rows itself
             h->wait_view = v;
             h->wait_ring = kernel == kSolveChain ? rv.chain.ring : 0;
         }
+    }
+    h->report.kernel = kernel == kSolveChain    ? CAPSP_KERNEL_CHAIN
+                       : kernel == kSolveStream ? CAPSP_KERNEL_STREAM
+                                                : CAPSP_KERNEL_ROW;
+    if (kernel == kSolveChain) {
+        h->report.ring = rv.chain.ring;
+        h->report.far_entries = rv.chain.far;
     }
     for (int r0 = 0; r0 < nrhs; r0 += 32) {
         const int nb = nrhs - r0 < 32 ? nrhs - r0 : 32;
@@ -1605,6 +1620,7 @@ static capsp_status_t enqueue_rows(capsp_handle_t h, int v, const T *b, T *x, in
         // ms, grad_1m 1.242 -> 1.230 ms), so FP32 walks the rows directly.
         const bool stage = level && nb == 1 && !wide_levels(h, v) && sizeof(T) == 8;
         CAPSP_CUDA(launch_row_solve<T>(a, kind, tn.R, blk, bps, h->num_sms, cap, stage, st));
+        h->report.launches += 2;
         if (prof)
             CAPSP_CUDA(cudaEventRecord(h->ev_k1, st));
     }
@@ -1669,6 +1685,7 @@ static capsp_status_t enqueue_cols(capsp_handle_t h, const T *b, T *x, int nrhs,
         const int cblock = tn.dflt ? (cnarrow && (nb > 1 || grad == nullptr) ? 128 : 256) : tn.block;
         const int cbps = tn.dflt ? 3 : tn.bps;
         CAPSP_CUDA(launch_col_solve<T>(a, cblock, cbps, h->num_sms, st));
+        h->report.launches++;
         if (prof)
             CAPSP_CUDA(cudaEventRecord(h->ev_k1, st));
     }
@@ -1695,7 +1712,9 @@ template <typename T>
 static capsp_status_t enqueue_op(capsp_handle_t h, Op op, const T *in, T *out, const T *xf, T *grad,
                                  int nrhs, int64_t ld, const Tuning &tn, cudaStream_t st)
 {
+    h->report = capsp_solve_report_t();
     if (column_driven(h, op)) {
+        h->report.kernel = CAPSP_KERNEL_COLUMN;
         // CSC solve (forward for lower) or CSR transpose (backward for lower),
         // with the gradient fused into the CSR transpose
         const int backward = op != kOpSolve ? (h->uplo == CAPSP_LOWER) : (h->uplo == CAPSP_UPPER);
@@ -1704,6 +1723,8 @@ static capsp_status_t enqueue_op(capsp_handle_t h, Op op, const T *in, T *out, c
     CAPSP_TRY(enqueue_rows<T>(h, view_of(h, op), in, out, nrhs, ld, tn, st));
     if (op == kOpTransposeGrad)
         CAPSP_TRY(enqueue_grad<T>(h, out, xf, grad, nrhs, ld, st));
+    if (op == kOpTransposeGrad)
+        h->report.launches += (nrhs + 31) / 32;
     return CAPSP_OK;
 }
 
@@ -2324,14 +2345,31 @@ extern "C" capsp_status_t capsp_get_info(capsp_handle_t h, capsp_info_t *info)
         } else if (kernel_wanted(h, v, tn, 1) == kSolveChain ||
                    (kernel_wanted(h, v, tn, 1) == kSolveStream && h->view[v].stream.ok)) {
             // these kernels need no selector table on the device; report
-            // the row kernels' choice for this matrix
-            std::vector<int> table((size_t)h->n + 2);
-            info->mix_len = capsp_mix_table(h->n, h->view[v].h_lcum.data(), 0, 32, tn.border, table.data(),
-                                            &info->warp_occupy, &info->element_occupy);
-            alg = info->warp_occupy > 0.0 ? CAPSP_ALG_MIX : CAPSP_ALG_WRTFST;
+            // the row kernels' choice for this matrix (made once)
+            MixTable &mt = h->view[v].mix_info;
+            if (mt.len == 0 || mt.border != tn.border) {
+                std::unique_ptr<int[]> table(new (std::nothrow) int[(size_t)h->n + 2]);
+                if (!table)
+                    return fail(CAPSP_ERR_OOM, "host allocation of the selector table failed");
+                mt.len = capsp_mix_table(h->n, h->view[v].h_lcum.data(), 0, 32, tn.border, table.get(), &mt.wo, &mt.eo);
+                mt.border = tn.border;
+            }
+            info->mix_len = mt.len;
+            info->warp_occupy = mt.wo;
+            info->element_occupy = mt.eo;
+            alg = mt.wo > 0.0 ? CAPSP_ALG_MIX : CAPSP_ALG_WRTFST;
         }
         info->algorithm = alg;
     }
+    return CAPSP_OK;
+}
+
+extern "C" capsp_status_t capsp_last_solve(capsp_handle_t h, capsp_solve_report_t *report)
+{
+    if (!h || !report)
+        return fail(CAPSP_ERR_INVALID, "handle and report must be non-NULL");
+    std::lock_guard<std::recursive_mutex> lk(h->mu);
+    *report = h->report;
     return CAPSP_OK;
 }
 

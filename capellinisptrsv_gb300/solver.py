@@ -272,6 +272,14 @@ class TriangularSolver:
         N.check(N.lib.capsp_get_info(self._h, C.byref(inf)))
         return {f: getattr(inf, f) for f, _ in N.Info._fields_}
 
+    def last_solve(self) -> dict:
+        """What the latest solve (of either kind) enqueued: kernel ("row", "chain", "stream",
+        "column"), kernels launched, and the chain kernel's ring and whether entries lie beyond it."""
+        r = N.SolveReport()
+        N.check(N.lib.capsp_last_solve(self._h, C.byref(r)))
+        return {"kernel": ("none", "row", "chain", "stream", "column")[r.kernel], "launches": r.launches,
+                "ring": r.ring, "far_entries": bool(r.far_entries)}
+
     def set_values(self, val) -> None:
         """Replace the values (same structure); refreshes 1/diag."""
         if self.on_device:

@@ -118,8 +118,10 @@ typedef struct capsp_info {
     int dtype;
     int format;
     int uplo;
-    int algorithm;          /* algorithm the next plain solve will use (AUTO resolved once
-                               its selector table exists) */
+    int algorithm;          /* row-kernel algorithm of the next plain solve (AUTO resolved once
+                               its selector table exists, or where AUTO solves with the chain or
+                               stream kernel: as it would be resolved without those;
+                               capsp_last_solve names the kernel) */
     int mix_len;            /* entries of the mix virtual-warp table (0 until built) */
     double warp_occupy;     /* rows handled warp-per-row / n   (mix/spts_..._wrt.h:152-156) */
     double element_occupy;  /* nnz in warp-per-row rows / nnz */
@@ -134,6 +136,24 @@ typedef struct capsp_info {
                                captured solve depends on (scratch growth, new value pointer,
                                schedule, tuning, wait budget, debug hooks) drops them all */
 } capsp_info_t;
+
+/* The kernel of a solve. */
+typedef enum capsp_kernel {
+    CAPSP_KERNEL_NONE = 0,   /* nothing solved yet */
+    CAPSP_KERNEL_ROW = 1,    /* row kernels: thread or warp per row */
+    CAPSP_KERNEL_CHAIN = 2,  /* narrow levels, the dependency chain inside one SM */
+    CAPSP_KERNEL_STREAM = 3, /* wide levels, several right-hand sides */
+    CAPSP_KERNEL_COLUMN = 4  /* column-driven (CAPSP_ALG_SYNCFREE_CSC) */
+} capsp_kernel_t;
+
+/* What the latest solve, transpose solve or solve with gradient enqueued
+ * (capsp_last_solve); a replay by capsp_graph_solve counts as its capture. */
+typedef struct capsp_solve_report {
+    int kernel;      /* capsp_kernel_t */
+    int launches;    /* kernels launched: solves, fills of publication vectors, gradients */
+    int ring;        /* chain kernel: values in its ring, else 0 */
+    int far_entries; /* chain kernel: 1 when some dependencies lie beyond the ring */
+} capsp_solve_report_t;
 
 /* ------------------------------------------------------------------------ */
 /* 1. Native API                                                             */
@@ -180,6 +200,9 @@ capsp_status_t capsp_refresh_values(capsp_handle_t h, const void *val, void *str
 capsp_status_t capsp_destroy(capsp_handle_t h);
 
 capsp_status_t capsp_get_info(capsp_handle_t h, capsp_info_t *info);
+
+/* Kernel and launches of the latest solve. */
+capsp_status_t capsp_last_solve(capsp_handle_t h, capsp_solve_report_t *report);
 
 /* L2 treatment of the publication vector of level-schedule row solves
  * (capsp_l2_policy_t).  The window modes reserve a persisting L2 carve-out of

@@ -97,6 +97,7 @@ _SIGS = {
     "capsp_last_kernel_ms": (I, [H, C.POINTER(C.c_float)]),
     "capsp_device_sms": (I, [IP]),
     "capsp_debug_set_stuck_row": (I, [H, I, C.c_uint64]),
+    "capsp_debug_set_stream_tickets": (I, [H, I]),
     "capsp_debug_trace": (I, [H, P]),
     "capsp_hop_latency": (I, [I, I, I, C.POINTER(C.c_float)]),
     "capsp_csc_solve_noalloc_f64": (I, [P, P, P, I, I, P, P, P]),

@@ -189,6 +189,7 @@ struct capsp_handle_s {
     // 7 % faster on deep chains (zipf_1m), where it delays each detection
     WaitCfg wait = {10000000000ull, 1u << 30, 0u};
     int stuck_row = -1;
+    bool stream_tickets = false;
     Graphs graphs;  // capsp_graph_solve; invalidated by every change a capture bakes in
     void *d_stage = nullptr;
     size_t stage_bytes = 0;
@@ -1061,6 +1062,16 @@ extern "C" capsp_status_t capsp_debug_set_stuck_row(capsp_handle_t h, int row, u
     return CAPSP_OK;
 }
 
+extern "C" capsp_status_t capsp_debug_set_stream_tickets(capsp_handle_t h, int enable)
+{
+    if (!h)
+        return fail(CAPSP_ERR_INVALID, "handle is NULL");
+    std::lock_guard<std::recursive_mutex> lk(h->mu);
+    h->stream_tickets = enable != 0;
+    h->graphs.invalidate();
+    return CAPSP_OK;
+}
+
 // ---------------------------------------------------------------------------
 // lazily built analysis products (never called while a stream is captured
 // for the first time: prepare() runs them before capture)
@@ -1389,6 +1400,10 @@ static capsp_status_t enqueue_stream(capsp_handle_t h, int v, const T *b, T *x, 
     const int cols = lanes_for_rhs(nb);
     CAPSP_CUDA(launch_fill_pending<T>((T *)sp.d_pub, 8 * sp.nslices, cols, cols, h->d_ticket, 3,
                                       first ? h->d_err : nullptr, st));
+    if (h->stream_tickets) {
+        static const unsigned tickets = kStreamTickets;
+        CAPSP_CUDA(cudaMemcpyAsync(h->d_ticket + 2, &tickets, sizeof(tickets), cudaMemcpyHostToDevice, st));
+    }
     StreamArgs<T> a;
     a.slice = sp.d_slice;
     a.npos = 8LL * sp.nslices;

@@ -123,6 +123,9 @@ struct ChainArgs {
     int stuck_row;
 };
 
+// how the stream kernel's warps share out the chunks (kernels_stream.cuh)
+enum { kStreamUndecided = 0, kStreamTurns = 1, kStreamTickets = 2 };
+
 // A row that the stream kernel passes over (debug hook), as its layout names it; and back
 #ifdef __CUDACC__
 __host__ __device__
@@ -143,7 +146,7 @@ struct StreamArgs {
     T *x;
     long long ld;
     int nrhs;           // <= 32
-    unsigned *words;    // three, zeroed before the launch
+    unsigned *words;    // tickets, blocks that run, the decision (kStream...); zeroed before the launch
     int *err;
     WaitCfg wait;
 };

@@ -124,7 +124,6 @@ struct StreamRow {
 // the last one to start says so).  kStreamTickets: a ticket per chunk, where some
 // block is not running yet, say behind another stream's work, after
 // kStreamStartNs.
-enum { kStreamUndecided = 0, kStreamTurns = 1, kStreamTickets = 2 };
 constexpr unsigned long long kStreamStartNs = 20000;
 
 // words[0]: tickets, [1]: blocks that run, [2]: the decision

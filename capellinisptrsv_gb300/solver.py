@@ -259,6 +259,9 @@ class TriangularSolver:
     def debug_stuck_row(self, row: int, timeout_s: float = 0.0) -> None:
         N.check(N.lib.capsp_debug_set_stuck_row(self._h, int(row), int(timeout_s * 1e9)))
 
+    def debug_stream_tickets(self, enable: bool) -> None:
+        N.check(N.lib.capsp_debug_set_stream_tickets(self._h, int(enable)))
+
     def trace(self, buf=None) -> None:
         """Per-row timing trace into a CUDA int64 tensor of 4*n entries (None: off)."""
         N.check(N.lib.capsp_debug_trace(self._h, _ptr(buf)))

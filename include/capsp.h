@@ -327,6 +327,10 @@ capsp_status_t capsp_device_sms(int *num_sms);
  * CAPSP_ERR_TIMEOUT.  row = -1 restores normal operation. */
 capsp_status_t capsp_debug_set_stuck_row(capsp_handle_t h, int row, uint64_t timeout_ns);
 
+/* Debug/testing: the stream kernel's warps take tickets, as they do by themselves
+ * where its blocks do not all start together.  enable = 0 restores that. */
+capsp_status_t capsp_debug_set_stream_tickets(capsp_handle_t h, int enable);
+
 /* Measure the per-hop dependency latency: solves a chain matrix where row i
  * depends on row i - stride (stride 1: neighbouring lanes of one warp;
  * stride 32*k: different warps) and returns the solve time divided by the

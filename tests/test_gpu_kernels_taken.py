@@ -8,6 +8,7 @@ import pytest
 import capellinisptrsv_gb300 as cs
 import oracle
 from conftest import rel_inf_err
+from test_gpu_stream import MATRICES as STREAMS
 from test_gpu_stream import blocks, dev, host
 
 torch = pytest.importorskip("torch")
@@ -93,3 +94,23 @@ def test_kernels_by_shape_and_algorithm():
     assert s.last_solve()["kernel"] == "row"  # one right-hand side on levels of 701 rows
     # "auto" before and after the first solve: the row kernels' choice
     assert s.info()["algorithm"] == 1
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("name", ["wide_short", "wide_batch_edges", "narrow_medium", "one_level"])
+def test_stream_tickets_give_what_turns_give(name, dtype):
+    """The share-out that is used where the blocks do not start together."""
+    make, ks = STREAMS[name]
+    m = make()
+    v = m.val.astype(dtype)
+    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(v))
+    for k in ks:
+        b = dev(np.random.default_rng(k).standard_normal((m.n, k)).astype(dtype))
+        s.debug_stream_tickets(False)
+        x = host(s.solve(b)).copy()
+        taken = s.last_solve()["kernel"]
+        s.debug_stream_tickets(True)
+        assert np.array_equal(host(s.solve(b)), x), k
+        # 33 go as 32 and one: the kernel is chosen for the 32
+        assert taken == s.last_solve()["kernel"] == "stream", (k, taken)
+    s.status()

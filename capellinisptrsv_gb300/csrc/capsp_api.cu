@@ -463,7 +463,7 @@ static ChainPlan plan_chain(int n, int levels, size_t vb, bool late, const int *
                             std::vector<int> &lnear)
 {
     ChainPlan c;
-    if (!chain_levels(n, levels))
+    if (!chain_levels(n, levels, lptr[n], vb == 8))
         return c;
     const bool deep = (long long)n < 64LL * (long long)levels;
     c.ring = 1024;

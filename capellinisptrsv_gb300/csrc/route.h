@@ -9,11 +9,21 @@ enum SolveKernel { kSolveRows = 0, kSolveChain = 1, kSolveStream = 2 };
 
 // Rows per level up to which the chain kernel is the faster one.  Measured on
 // GB300 in FP64, chain against row kernel: 8 rows per level (1,048,576 Zipf rows)
-// 28.3 against 100.9 ms, 13 (2,003 rows) 27 against 137 us, 115 (40,000 rows of
+// 28.4 against 100.9 ms, 13 (2,003 rows) 29 against 137 us, 115 (40,000 rows of
 // 3-12 dependencies) 162 against 460 us, 146 (38,261 rows of 3-10) 146 against 336
 // us, 200 (20,000 rows of 1-5) 57 against 92 us, 377 (60,000 rows of 1-7) 171
 // against 147 us.
 constexpr long long kChainLevelRows = 256;
+// ... and off-diagonal entries per level, as one SM walks them all.  Time of the row
+// kernel / time of the chain kernel on 150 levels (rows per level, mean entries: 1, 4,
+// 16 and 32 right-hand sides):
+//   FP64  200 x 24  1.35 1.04 1.11 1.48    150 x 34  1.37 1.07 1.24 1.74
+//         256 x 14  1.25 1.39 1.28 1.92    240 x 21  1.42 1.51 1.48 2.20
+//         240 x 24  1.00 0.83 0.90 1.25    180 x 34  1.19 0.91 1.06 1.50
+//         256 x 26  0.96 0.93 0.94 1.65    256 x 34  0.86 0.60 0.73 1.05
+//   FP32  256 x 34  1.97 1.33 1.51 2.39    240 x 48  1.37 1.02 1.30 2.21
+//         256 x 48  1.09 0.79 1.01 1.77
+constexpr long long kChainLevelEntries64 = 5120, kChainLevelEntries32 = 11520;
 
 // Rows per level below which the row kernels give every row a warp
 constexpr long long kDeepRows = 32;
@@ -44,7 +54,10 @@ struct ViewShape {
 };
 
 // whether the levels are narrow enough for the chain kernel
-inline bool chain_levels(long long n, long long levels) { return n <= kChainLevelRows * levels; }
+inline bool chain_levels(long long n, long long levels, long long entries, bool f64)
+{
+    return n <= kChainLevelRows * levels && entries <= (f64 ? kChainLevelEntries64 : kChainLevelEntries32) * levels;
+}
 
 // `cols`: right-hand sides, rounded up to the lanes or lane slots they take.
 //

@@ -23,7 +23,7 @@ static ViewShape shape(long long rows, long long levels, long long mean, int lon
     s.entries = mean * s.n;
     s.longest = longest;
     s.f64 = f64;
-    s.chain = chain_levels(s.n, s.levels);  // as where the plan fits
+    s.chain = chain_levels(s.n, s.levels, s.entries, f64);  // as where the plan fits
     return s;
 }
 
@@ -46,7 +46,10 @@ int main()
                 // rows longer than a lane walks
                 CHECK(auto_kernel(shape(20000, 3, mean, 129, f64), cols) == kSolveRows);
             }
-    CHECK(!chain_levels(25601, 100) && chain_levels(25600, 100));
+    CHECK(!chain_levels(25601, 100, 0, true) && chain_levels(25600, 100, 0, true));
+    // entries per level, by precision
+    CHECK(chain_levels(20000, 100, 512000, true) && !chain_levels(20000, 100, 512001, true));
+    CHECK(chain_levels(20000, 100, 1152000, false) && !chain_levels(20000, 100, 1152001, false));
     // two right-hand sides, and FP64 by row-columns per level
     CHECK(auto_kernel(shape(8191, 3, 4, 12, true), 2) == kSolveRows);
     CHECK(auto_kernel(shape(8192, 3, 4, 12, true), 2) == kSolveStream);

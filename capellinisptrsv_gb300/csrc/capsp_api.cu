@@ -1439,8 +1439,11 @@ static capsp_status_t enqueue_stream(capsp_handle_t h, int v, const T *b, T *x, 
     const bool pairs = cols >= 4 && per_level * cols >= (sizeof(T) == 8 ? 65536 : 32768);
     // few elements per level: fewer warps, whose polls disturb each other less
     // (FP64, 1,000 rows per level: 4 RHS 986 us with 8 warps, 1,028 with 12, 1,110
-    // with 16; 16 RHS 1,100, 1,004 and 1,050 us; 750 rows, 16 RHS: 513 and 433 us)
-    const int warps = per_level * cols < 10240 ? 8 : per_level * cols < 20480 ? 12 : 32;
+    // with 16; 16 RHS 1,100, 1,004 and 1,050 us; 750 rows, 16 RHS: 513 and 433 us).
+    // 12 against all of them: 1,500 rows of 2, 16 RHS 161 against 182 us (row kernel
+    // 167), 3,000 of 2, 8 RHS 170 against 189 (181), 3,500 of 12, 8 RHS 229 against 253,
+    // 7,000 of 11, 4 RHS 129 against 145; FP32 3 to 9 % less too
+    const int warps = per_level * cols < 10240 ? 8 : per_level * cols < 28672 ? 12 : 32;
     CAPSP_CUDA(launch_stream_solve<T>(a, long_rows, pairs, warps, h->num_sms, st));
     h->report.launches += 2;
     if (prof)

@@ -18,6 +18,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -560,13 +561,12 @@ static capsp_status_t build_stream(capsp_handle_t h, RowView &rv)
     sp.nslices = capsp_stream_slices(rv.levels, rv.h_levels.data());
     const size_t ns = sp.nslices > 0 ? (size_t)sp.nslices : 0;
     std::unique_ptr<int[]> rec(new (std::nothrow) int[2 * ns + 1]), pos(new (std::nothrow) int[8 * ns + 1]);
-    if (!rec || !pos)
-        return fail(CAPSP_ERR_OOM, "host allocation failed while laying out slices");
     long long entries = LLONG_MAX;
-    if (sp.nslices > 0)
+    if (sp.nslices > 0 && rec && pos) {
         entries = capsp_stream_layout(rv.levels, rv.h_levels.data(), rv.h_lcum.data(), 1, rec.get(), pos.get());
-    if (entries < 0)
-        return fail(CAPSP_ERR_OOM, "host allocation failed while laying out slices");
+        if (entries < 0)
+            entries = LLONG_MAX;  // no host memory: the row kernels do without
+    }
     if (entries > INT_MAX || entries > 2 * ((long long)h->nnz - h->n) + 256LL * rv.levels) {
         rv.stream = sp;
         return CAPSP_OK;
@@ -616,7 +616,7 @@ static capsp_status_t build_stream(capsp_handle_t h, RowView &rv)
 // Build the level schedule of view v (host work O(nnz) plus one upload);
 // synchronous.
 static capsp_status_t build_view(capsp_handle_t h, int v)
-{
+try {
     RowView &rv = h->view[v];
     if (rv.built)
         return CAPSP_OK;
@@ -690,8 +690,12 @@ static capsp_status_t build_view(capsp_handle_t h, int v)
     rv.chain = plan_chain(n, levels, vb, late, lptr.data(), lidx.data(), lnear);
     cudaFree(rv.d_lnear);
     rv.d_lnear = nullptr;
+    if (rv.chain.ok && cudaMalloc(&rv.d_lnear, sizeof(int) * (size_t)n) != cudaSuccess) {
+        cudaGetLastError();
+        rv.d_lnear = nullptr;
+        rv.chain.ok = false;  // no room: the row kernels do without
+    }
     if (rv.chain.ok) {
-        CAPSP_CUDA(cudaMalloc(&rv.d_lnear, sizeof(int) * (size_t)n));
         CAPSP_CUDA(cudaMemcpy(rv.d_lnear, lnear.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice));
     }
     rv.h_levels.assign(level_start.begin() + 1, level_start.begin() + levels + 2);
@@ -716,6 +720,8 @@ static capsp_status_t build_view(capsp_handle_t h, int v)
     if (auto_kernel(view_shape(h, rv, 1), 1) == kSolveStream)
         return build_stream(h, rv);
     return CAPSP_OK;
+} catch (const std::bad_alloc &) {
+    return fail(CAPSP_ERR_OOM, "host allocation failed while building the level schedule");
 }
 
 extern "C" capsp_status_t capsp_device_sms(int *num_sms)

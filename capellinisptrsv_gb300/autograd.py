@@ -1,7 +1,7 @@
 """Differentiable sparse triangular solve: x = L^{-1} b as a torch.autograd.Function.
 
 Forward runs the row-driven sync-free solve.  Backward is hand-written: the
-same row kernels over the solver's transposed copy of the structure (built
+same kernels over the solver's transposed copy of the structure (built
 once, its entries pointing back into the CSR values) solve L^T y = g
 (grad_b = y), then one pass writes grad_val[k] = -sum_r y[row_k, r] *
 x[col_k, r] for every stored entry k, each sum over the right-hand sides an

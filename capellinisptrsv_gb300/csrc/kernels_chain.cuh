@@ -23,7 +23,7 @@
 // diverge 300), and a row's dependencies that land together cost a round each.
 // 1,048,576 Zipf rows in 126k levels: 100.9 ms with the row kernel (0.79 us per
 // level), 28.3 ms here (0.22 us); 131,072 rows of 40 dependencies in 87k
-// levels: 64.7 -> 10.7 ms; 2,003 rows in 153 levels: 137 -> 27 us (one launch
+// levels: 64.7 -> 10.7 ms; 2,003 rows in 153 levels: 137 -> 29 us (one launch
 // instead of two); 20,000 rows in 100 levels: 92 -> 53 us.
 //
 // Per round a lane loads its next dependency's ring value together with that

@@ -9,7 +9,7 @@ enum SolveKernel { kSolveRows = 0, kSolveChain = 1, kSolveStream = 2 };
 
 // Rows per level up to which the chain kernel is the faster one.  Measured on
 // GB300 in FP64, chain against row kernel: 8 rows per level (1,048,576 Zipf rows)
-// 28.4 against 100.9 ms, 13 (2,003 rows) 29 against 137 us, 115 (40,000 rows of
+// 28.3 against 100.9 ms, 13 (2,003 rows) 29 against 137 us, 115 (40,000 rows of
 // 3-12 dependencies) 162 against 460 us, 146 (38,261 rows of 3-10) 146 against 336
 // us, 200 (20,000 rows of 1-5) 57 against 92 us, 377 (60,000 rows of 1-7) 171
 // against 147 us.
@@ -40,8 +40,10 @@ constexpr int kStreamLongest = 128;
 // lane one entry after the other; where such rows are the norm that shows (12,800 rows
 // per level, 33-60 entries, 2-norm of the error against more than 64 bits: FP64 2.6e-17,
 // in a lane 4.6e-17; FP32 1.4e-8, 2.4e-8), where they are few it is lost in the rest
-// (a seventh or a sixth of the rows: 1.02 to 1.06 times the error).  With 8 and more
-// the row kernels use a lane too.
+// (a seventh or a sixth of the rows: 1.02 to 1.06 times the error).  The trees cost
+// time: 12,288 rows per level, 26 entries on average, FP64, row kernels / stream kernel
+// 203 / 61 us (1 RHS) and 151 / 65 us (4); 6,000 rows of 33, FP32, 4 RHS 154 / 77 us; 1,500
+// rows of 64 195 / 194 us.  With 8 and more the row kernels use a lane too.
 constexpr long long kStreamHeavyShare = 6;
 constexpr int kHeavyEntries = 32;  // stored entries per row of such a group, on average
 

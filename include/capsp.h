@@ -81,8 +81,10 @@ typedef enum capsp_uplo {
  * other orientation column by column on the stored arrays. */
 typedef enum capsp_algorithm {
     CAPSP_ALG_AUTO = 0,        /* level schedule with levels of up to 256 rows on average: the chain kernel
-                                  (the dependency chain inside one SM); else mix when the selector
-                                  finds heavy row groups, else WRTFST */
+                                  (the dependency chain inside one SM), unless its rows are long; wide
+                                  levels, and several right-hand sides on narrower ones: the stream
+                                  kernel; else mix when the selector finds heavy row groups, else
+                                  WRTFST.  capsp_last_solve names the kernel that ran */
     CAPSP_ALG_WRTFST = 1,      /* thread per row, write-first (CUDA/ourWrtFst) */
     CAPSP_ALG_TWOPART = 2,     /* thread per row, out-of-warp then in-warp phases (CUDA/our2Part) */
     CAPSP_ALG_MIX = 3,         /* thread or warp per row by nnz/row of 32-row groups (CUDA/mix) */
@@ -178,6 +180,8 @@ capsp_status_t capsp_analyse(int n, int nnz, const int *ptr, const int *idx,
  * concatenated matrix with GLOBAL indices; sys_rowoff[nsys+1] gives the first
  * row of every system (sys_rowoff[0] = 0, sys_rowoff[nsys] = n).  The result
  * is an ordinary handle: capsp_solve solves every system in one launch.
+ * Levels of 4,096 rows and more (all systems together) get the stream layout here,
+ * as if capsp_reserve had been called for 4 right-hand sides.
  * No reference counterpart (the reference solves one system per process). */
 capsp_status_t capsp_batched_create(int nsys, const int *sys_rowoff, int n, int nnz,
                                     const int *ptr, const int *idx, const void *val,
@@ -243,6 +247,12 @@ capsp_status_t capsp_set_backoff(capsp_handle_t h, unsigned sleep_max_ns);
 /* Solve op(A) X = B for nrhs right-hand sides (device pointers, element
  * (i,r) at i*ld + r, ld >= nrhs).  x must not alias b.  Stream-ordered,
  * no host synchronisation, no allocation once capsp_reserve covered nrhs.
+ * Without that, the first solve that AUTO gives to the stream kernel builds its
+ * layout: host passes over the rows, one allocation, two synchronisations of the
+ * device.  The layout holds every entry a second time (index, source, value: 16
+ * bytes in FP64, 12 in FP32, padded to slices of 8 rows) and 17 (13) bytes per row,
+ * beside a publication vector of its own; where there is no memory for it the row
+ * kernels solve.
  * Replaces the timed launch of spts_syncfree_cuda_executor_csr_wrt
  * (CUDA/ourWrtFst/spts_syncfree_cuda_csr_wrt.h:10-57,160), of
  * spts_syncfree_cuda_executor_csr (CUDA/our2Part/spts_syncfree_cuda_csr.h:10-124),
@@ -268,13 +278,14 @@ capsp_status_t capsp_grad_val(capsp_handle_t h, const void *y, const void *x,
 
 /* Backward of x = L^{-1} b: y = L^{-T} g (as capsp_solve_transpose), then
  * grad_val as capsp_grad_val; under CAPSP_ALG_SYNCFREE_CSC a CSR handle fuses
- * grad_val into its column-driven stream.  No reference counterpart. */
+ * grad_val into its column-driven sweep.  No reference counterpart. */
 capsp_status_t capsp_solve_transpose_grad(capsp_handle_t h, const void *g,
                                           const void *x, void *y, void *grad_val,
                                           int nrhs, int64_t ld, void *stream);
 
-/* Pre-allocate per-handle scratch for up to max_nrhs right-hand sides so later
- * solves (and CUDA-graph captures of them) allocate nothing. */
+/* Pre-allocate per-handle scratch for up to max_nrhs right-hand sides, and build the
+ * transposed view and the layouts that the handle's algorithm takes for them, so that
+ * later solves (and CUDA-graph captures of them) build and allocate nothing. */
 capsp_status_t capsp_reserve(capsp_handle_t h, int max_nrhs);
 
 /* Synchronise `stream` and report the device-side status of the latest

@@ -685,7 +685,7 @@ try {
     rv.upper = upper;
     rv.levels = levels;
     std::vector<int> lnear;
-    // where the row kernels give every row, or most, a warp (untuned) and sum it as a tree
+    // where the row kernels give every row, or many rows, a warp (untuned) and sum them as trees
     const bool late = n < kDeepRows * levels || kStreamHeavyShare * rv.heavy[0] > n;
     rv.chain = plan_chain(n, levels, vb, late, lptr.data(), lidx.data(), lnear);
     cudaFree(rv.d_lnear);

@@ -1842,7 +1842,9 @@ static capsp_status_t prepare(capsp_handle_t h, int nrhs, Op op)
         }
         CAPSP_TRY(ensure_xp(h, nrhs));  // fewer right-hand sides may go to the row kernels
     }
-    if ((tn.kind == kRowMix || tn.kind < 0) && kernel == kSolveRows) {
+    // (a captured solve with a row that never publishes takes the row kernels too)
+    if ((tn.kind == kRowMix || tn.kind < 0) &&
+        (kernel == kSolveRows || (kernel == kSolveStream && h->stuck_row >= 0))) {
         MixTable *mt = nullptr;
         for (int r0 = 0; r0 < nrhs; r0 += 32) {
             const int nb = nrhs - r0 < 32 ? nrhs - r0 : 32;

@@ -46,6 +46,26 @@ def test_stream_reports_the_waiting_row(k):
     check(m, reported(m, s, b, stuck), stuck)
 
 
+def test_graph_replays_report_too():
+    """The hook inside the handle's own capture, where AUTO otherwise takes the stream kernel."""
+    m = blocks(6, 12_301, 3, 11, 12)
+    b = np.random.default_rng(2).standard_normal((m.n, 4))
+    s = cs.TriangularSolver(dev(m.rowptr), dev(m.colidx), dev(m.val))
+    st = torch.cuda.Stream()
+    bd = dev(b)
+    x = torch.empty_like(bd)
+    torch.cuda.synchronize()
+    s.debug_stuck_row(int(m.colidx[m.rowptr[15_000]]), timeout_s=0.02)
+    s.graph_solve(bd, x, st)
+    with pytest.raises(cs.CapspError) as e:
+        s.status(st)
+    assert e.value.status == 2
+    s.debug_stuck_row(-1, timeout_s=10.0)
+    s.graph_solve(bd, x, st)
+    s.status(st)
+    assert rel_inf_err(host(x), oracle.solve_csr_lower(m.rowptr, m.colidx, m.val, b)) <= 1e-12
+
+
 CHAINS = {
     # near entries only; far entries, folded by a lane or by a warp; entries walked in global memory
     "near": lambda: cs.generate(n=1_025, kmin=1, kmax=6, band=60, seed=3),
